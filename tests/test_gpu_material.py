@@ -223,3 +223,27 @@ def test_elastoplastic_host_entry_equals_device_entry():
     assert rc == st[0]
     assert np.array_equal(hs.T, s1) and np.array_equal(hz, z1) and np.array_equal(he, el1)
     assert np.array_equal(c2, c1) and np.array_equal(n2, n1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ndim", [2, 3])
+@pytest.mark.parametrize("n", [1, 33, 80001])
+def test_elastoplastic_lanes_take_the_next_points(ndim, n):
+    """Sizes below, at the edge of and beyond one point per lane of a full grid (its lanes then take
+    further points as they finish), ragged last runs included: the oracle's cases, failures and states
+    (1e-8 of the largest stress, as for the seeded states above)."""
+    import ep_cases as E
+    sig, z, deps = E.random_states(n, ndim, seed=91 + ndim)
+    prm = oracle.Params(E.YOUNG, E.POISSON, E.HH, E.Z_INI)
+    osig, oz, oel = sig.copy(), z.copy(), np.zeros(n, dtype=np.uint8)
+    _, ocases, osteps, _ = oracle.ep_update(prm, ndim, osig, oz, oel, deps)
+    s1, z1, el, cases, steps, _ = _ep_device(ndim, sig, z, deps)
+    assert np.array_equal(cases < 0, ocases < 0)
+    off = np.abs(np.array([E.sigma_d(v) for v in sig]) - z) > 1e-12 * z  # not on the surface up to rounding
+    assert np.array_equal(cases[off], ocases[off])
+    same = cases >= 0
+    assert np.array_equal(el[same], oel[same])
+    scale = max(np.abs(osig).max(), E.Z_INI)
+    assert np.abs(s1 - osig)[same].max(initial=0.0) <= 1e-8 * scale
+    assert np.abs(z1 - oz)[same].max(initial=0.0) <= 1e-8 * scale
+    assert np.array_equal(s1[~same], sig[~same]) and np.array_equal(z1[~same], z[~same])
