@@ -184,8 +184,8 @@ int pms_elements_set_symmetry(pms_elements* h, int32_t sym);
 
 /* Instrumentation: when on, every batched call records CUDA events around its kernels on the
  * handle's stream; pms_elements_kernel_times waits for the stream and returns the summed device
- * time (ms) and launch count of [0] element kernel, [1] F_int gather, [2] CSR gather since the
- * previous query. */
+ * time (ms) and launch count of [0] element kernel, [1] F_int gather (calls that ask for no K: the
+ * CSR gather forms F_int as well), [2] CSR gather since the previous query. */
 int pms_elements_set_timing(pms_elements* h, int32_t on);
 int pms_elements_kernel_times(pms_elements* h, double* ms, int64_t* counts);
 

@@ -44,6 +44,7 @@
 
 #include "../../include/pms.h"
 #include "pms_device.cuh"
+#include "pms_gather.h"
 #include "pms_internal.h"
 #include "pms_pattern.h"
 #include "pms_shapes.h"
@@ -90,8 +91,8 @@ struct ElemArgs {
     // dense outputs (no CSR): the fe / ke rows of cell c are c - ke_cell0
     int64_t ke_cell0 = 0;
     // ke layout: 0 = full row-major NE x NE (per-cell calls); 1 = the upper node-pair blocks (a <= b)
-    // only: block row a holds its ND scalar rows one after another, each with the columns of nodes
-    // a..NN-1 (upper_entry), NN(NN+1)/2 ND x ND blocks per cell (the gather assembly)
+    // only, row by row, each ND x ND block contiguous (upper_entry): NN(NN+1)/2 blocks per cell (the
+    // gather assembly)
     int ke_upper = 0;
     // direct assembly (CSR kernels): cell c adds its node-row slab a into block row A = conn[c][a]
     // and its F_int share into R once ticket[A] equals c's rank among A's cells (crank), then
@@ -137,15 +138,6 @@ __device__ __forceinline__ int64_t dequeue(unsigned long long* next) {
 // issuing lane does not wait.  The row tickets order the adds of successive cells (each cell's
 // adds come after the release store that the next cell acquires), so every entry is still summed
 // in ascending cell order.
-// Number of node-pair blocks (a', b'), a' <= b', in the block rows before row a (upper layout).
-__host__ __device__ constexpr int upper_block(int nn, int a, int b) { return a * nn - a * (a - 1) / 2 + (b - a); }
-// Upper layout of an element matrix: entry (i, j) of block (a, b), a <= b, at
-// BB*upper_block(a, a) + i*(NN - a)*ND + (b - a)*ND + j (block row a, scalar rows one after another).
-template <int NN, int ND>
-__host__ __device__ constexpr int upper_entry(int a, int b, int i, int j) {
-    return ND * ND * upper_block(NN, a, a) + i * (NN - a) * ND + (b - a) * ND + j;
-}
-
 // Asynchronous global -> shared copies (no register passes through; cp.async.wait_all, then a warp
 // barrier, before the data is read).  Sizes 4, 8 and 16 bytes, both addresses aligned to the size.
 template <int B>
@@ -1551,8 +1543,8 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
                             if (up) {
 #pragma unroll
                                 for (int i = 0; i < 2; i++)
-#pragma unroll
-                                    for (int j = 0; j < 2; j++) stage[upper_entry<NN, 2>(a, b, i, j)] = acc[r][c][i][j];
+                                    *reinterpret_cast<double2*>(stage + upper_entry<NN, 2>(a, b, i, 0)) =
+                                        make_double2(acc[r][c][i][0], acc[r][c][i][1]);
                             } else {
 #pragma unroll
                                 for (int i = 0; i < 2; i++)
@@ -1703,185 +1695,14 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
     }
 }
 
-// One warp per G = 32/NN consecutive block rows of K (a work-queue range may cut the run); group g
-// of NN lanes owns row A_g.  Lane b of the group loads, for each incidence k of A_g (cell c, local
-// index a), the ND x ND block (a, b) of c's element matrix -- kept as its upper blocks, block row by
-// block row, so lane b reads block (a, b) when a <= b (the lanes b >= a read adjacent segments of
-// the same scalar rows) and the transpose of block (b, a) otherwise -- and adds it at column
-// slot[k*NN + b] of the row's buffer in shared memory.  Up
-// to NB incidences are loaded before they are added; the adds go in ascending incidence (= cell)
-// order with a group barrier between incidences, so every entry of K is the fixed-order sum over
-// its cells: bit-identical on every run.  The G buffers lie back to back in CSR order, so when the
-// rows are consecutive the warp writes them out as one contiguous run.  Rows of problems whose mode
-// is 0 are skipped (per-problem batches).
-template <int ND, int NN> struct GatherShape {
-    static constexpr int G = NN >= 32 ? 1 : 32 / NN;  // rows per warp
-    static constexpr int NB = 4;                      // incidences loaded before they are added
-};
-
-// TRI: the CSR values hold one triangle of K (sym = PMS_SYM_LOWER: columns <= row, PMS_SYM_UPPER:
-// columns >= row; src/base/assembly.rs:92-122): the lanes skip the blocks that fall outside it, and
-// row (A, i) starts at tbase[A] plus the lengths of rows (A, 0..i-1); kdiag[A] = A's own position
-// in its block row.
-template <int ND, int NN, bool TRI>
-__global__ void __launch_bounds__(256, ND == 2 ? 4 : 1) kk_gather_kernel(int64_t npoint, int nbmax, const int64_t* __restrict__ bptr,
-                                                        const int64_t* __restrict__ inc_ptr,
-                                                        const int32_t* __restrict__ inc,
-                                                        const int16_t* __restrict__ slot,
-                                                        const double* __restrict__ ke, double* __restrict__ csr,
-                                                        const int32_t* __restrict__ node_prob,
-                                                        const uint8_t* __restrict__ pmode, int nq,
-                                                        const int64_t* __restrict__ q_off,
-                                                        const int64_t* __restrict__ q_first, int64_t node0,
-                                                        int sym, const int32_t* __restrict__ kdiag,
-                                                        const int64_t* __restrict__ tbase) {
-    constexpr int BB = ND * ND, NU = NN * (NN + 1) / 2;
-    constexpr int G = GatherShape<ND, NN>::G, NB = GatherShape<ND, NN>::NB;
-    extern __shared__ double rowbuf[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    double* buf = rowbuf + (int64_t)wid * G * nbmax * BB;
-    const int g = lane / NN, b = lane - (lane / NN) * NN;
-    const bool lane_on = g < G;
-    const unsigned gmask = lane_on ? (((NN >= 32) ? 0xffffffffu : ((1u << NN) - 1u)) << (g * NN)) : (1u << lane);
-    const int64_t ngroup = (npoint + G - 1) / G;
-    const int64_t nwarp = (int64_t)gridDim.x * wpb;
-    for (int64_t w = (int64_t)blockIdx.x * wpb + wid; w < ngroup; w += nwarp) {
-        const int64_t Ai = w * G + g;
-        bool on = lane_on && Ai < npoint;
-        int64_t A = 0;
-        if (on) {
-            A = nq ? queue_item(Ai, nq, q_off, q_first) : node0 + Ai;
-            if (pmode && pmode[node_prob[A]] == 0) on = false;
-        }
-        int64_t ba = 0;
-        int nba = 0, dp = 0;
-        if (on) {
-            ba = bptr[A];
-            nba = (int)(bptr[A + 1] - ba);
-            if constexpr (TRI) dp = kdiag[A];
-        }
-        // buffer offsets of the group rows (exclusive scan over the groups) and the run test
-        int off = 0, total = 0;
-#pragma unroll
-        for (int q = 0; q < G; q++) {
-            const int nq_ = __shfl_sync(FULL, nba, q * NN);
-            if (q < g) off += nq_;
-            total += nq_;
-        }
-        const int64_t A0 = __shfl_sync(FULL, A, 0);
-        const bool on0 = __shfl_sync(FULL, on, 0);
-        const bool fits = !lane_on || Ai >= npoint || (on && A == A0 + g);
-        const bool run = !TRI && __all_sync(FULL, fits) && on0;
-        for (int t = lane; t < total * BB; t += 32) buf[t] = 0.0;
-        __syncwarp();
-        if (on) {
-            double* rb = buf + (int64_t)off * BB;
-            const int nrow = ND * nba;
-            const int64_t k0 = inc_ptr[A], k1 = inc_ptr[A + 1];
-            for (int64_t kb = k0; kb < k1; kb += NB) {
-                double v[NB][BB];
-                int pos[NB];
-#pragma unroll
-                for (int r = 0; r < NB; r++) {
-                    const int64_t k = kb + r;
-                    pos[r] = -1;
-                    if (k < k1) {
-                        const int32_t code = __ldg(inc + k);
-                        const int64_t cell = code / NN;
-                        const int a = code - (int)cell * NN;
-                        pos[r] = __ldg(slot + k * NN + b);
-                        if constexpr (TRI) {
-                            if (sym == PMS_SYM_LOWER ? pos[r] > dp : pos[r] < dp) {
-                                pos[r] = -1;  // outside the stored triangle: neither loaded nor added
-#pragma unroll
-                                for (int i = 0; i < BB; i++) v[r][i] = 0.0;
-                                continue;
-                            }
-                        }
-                        // block (a, b) of the upper layout: stored as (a, b) when a <= b, else as (b, a);
-                        // the lanes b >= a read adjacent segments of the same scalar rows
-                        const bool upper = a <= b;
-                        const int lo = upper ? a : b, hi = upper ? b : a;
-                        const double* src = ke + cell * (int64_t)(NU * BB) + upper_entry<NN, ND>(lo, hi, 0, 0);
-                        const int rs = (NN - lo) * ND;  // scalar-row stride of block row lo
-#pragma unroll
-                        for (int i = 0; i < ND; i++)
-#pragma unroll
-                            for (int j = 0; j < ND; j++) v[r][i * ND + j] = __ldg(src + (upper ? i * rs + j : j * rs + i));
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < BB; i++) v[r][i] = 0.0;
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < NB; r++) {
-                    __syncwarp(gmask);  // the group's previous incidence is added
-                    if (pos[r] >= 0) {
-#pragma unroll
-                        for (int i = 0; i < ND; i++)
-#pragma unroll
-                            for (int j = 0; j < ND; j++) rb[i * nrow + pos[r] * ND + j] += v[r][i * ND + j];
-                    }
-                }
-            }
-        }
-        __syncwarp();
-        if (run) {
-            double* dst = csr + (int64_t)BB * __shfl_sync(FULL, ba, 0);
-            for (int t = lane; t < total * BB; t += 32) dst[t] = buf[t];
-        } else if constexpr (TRI) {
-            // buffer entry (i, c = p*ND + j) of a row group is K(A*ND + i, B_p*ND + j).  The group's
-            // stored entries are contiguous from tbase[A]: row i holds, lower, c = 0 .. ND*dq + i
-            // (from i*ND*dq + i(i+1)/2 on), upper, c = dq*ND + i .. ND*nq - 1 (from
-            // i*ND*(nq - dq) - i(i-1)/2 on); each lane takes destinations and finds their row
-            const bool lower = sym == PMS_SYM_LOWER;
-            const int64_t tb = on ? tbase[A] : 0;
-            int oq = 0;
-#pragma unroll 1
-            for (int q = 0; q < G; q++) {
-                const int nq_ = __shfl_sync(FULL, nba, q * NN);
-                const int dq = __shfl_sync(FULL, dp, q * NN);
-                double* dst = csr + __shfl_sync(FULL, tb, q * NN);
-                const double* src = buf + (int64_t)oq * BB;
-                const int nrow = ND * nq_, w = lower ? ND * dq : ND * (nq_ - dq);
-                const int cnt = nq_ ? (lower ? BB * dq : BB * (nq_ - dq - 1)) + ND * (ND + 1) / 2 : 0;
-                for (int u = lane; u < cnt; u += 32) {
-                    int i = 0, s0 = 0;
-#pragma unroll
-                    for (int ii = 1; ii < ND; ii++) {
-                        const int s = lower ? ii * w + ii * (ii + 1) / 2 : ii * w - ii * (ii - 1) / 2;
-                        if (u >= s) i = ii, s0 = s;
-                    }
-                    dst[u] = src[i * nrow + (u - s0) + (lower ? 0 : dq * ND + i)];
-                }
-                oq += nq_;
-            }
-        } else {
-            int oq = 0;
-#pragma unroll 1
-            for (int q = 0; q < G; q++) {
-                const int nq_ = __shfl_sync(FULL, nba, q * NN);
-                const int64_t bq = __shfl_sync(FULL, ba, q * NN);
-                double* dst = csr + (int64_t)BB * bq;  // rows that are absent or inactive have nq_ = 0
-                const double* src = buf + (int64_t)oq * BB;
-                for (int t = lane; t < nq_ * BB; t += 32) dst[t] = src[t];
-                oq += nq_;
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// One thread per point: R[A*nd + i] = sum over its incidences (ascending cell) of f_e.
+// R alone (no K asked for): one thread per point, R[A*nd + i] = sum over its incidences (ascending cell)
+// of f_e.
 template <int ND>
 __global__ void __launch_bounds__(256) f_gather_kernel(int64_t npoint, const int64_t* __restrict__ inc_ptr,
                                                        const int32_t* __restrict__ inc,
-                                                       const double* __restrict__ fe, double* __restrict__ ff,
-                                                       int nq = 0, const int64_t* __restrict__ q_off = nullptr,
-                                                       const int64_t* __restrict__ q_first = nullptr) {
-    for (int64_t Ai = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; Ai < npoint;
-         Ai += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t A = nq ? queue_item(Ai, nq, q_off, q_first) : Ai;
+                                                       const double* __restrict__ fe, double* __restrict__ ff) {
+    for (int64_t A = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; A < npoint;
+         A += (int64_t)gridDim.x * blockDim.x) {
         double s[ND];
 #pragma unroll
         for (int i = 0; i < ND; i++) s[i] = 0.0;
@@ -1916,7 +1737,6 @@ __global__ void zero_lambda_kernel(int64_t nip, double* lam) {
 // ------------------------------------------------------------------------------- handle
 struct pms_elements {
     int nd = 0, kind = 0, nn = 0, ng = 0, nc = 0;
-    int gather_wpb = 8, gather_smem = 0;  // rows (warps) per block and shared memory of kk_gather
     int64_t npoint = 0, ncell = 0, ndof = 0, nip = 0, nnz = 0;
     double thickness = 1.0;
     int axisym = 0;
@@ -1966,6 +1786,13 @@ struct pms_elements {
     int64_t launches = 0;
     int smem_bytes = 0;
     std::vector<void*> allocs;
+    // launch plans made so far: blocks of a kernel that the device holds at once (launch_plan)
+    struct Plan {
+        const void* kern;
+        int smem;
+        int64_t resident;
+    };
+    std::vector<Plan> plans;
     // host-memory calls: the CSR values leave in row slabs on copy_stream while later slabs gather
     static constexpr int NSLAB = 8;
     cudaStream_t copy_stream = nullptr;
@@ -2041,16 +1868,21 @@ int grid_1d(int64_t n) {
 }
 
 // Lets a kernel take up to the device's opt-in shared memory per block (each launch still asks for
-// its own size, from which the residency is computed).
-void allow_dynamic_smem(const void* kern) {
+// its own size, from which the residency is computed).  max_shared: no more L1 than the largest shared
+// memory leaves; else the driver sets the carveout to what the resident blocks need.
+void allow_dynamic_smem(const void* kern, bool max_shared = true) {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    if (max_shared)
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 
-// Blocks of a kernel that the GPU holds at once (one wave of the persistent element kernel).
-int64_t resident_blocks(const void* kern, int smem, int threads = WPB * 32) {
+// Blocks of a kernel that the GPU holds at once (one wave of a persistent kernel); sets the kernel's
+// attributes on the current device first.
+int64_t resident_blocks(const void* kern, int smem, int threads, bool max_shared = true) {
+    allow_dynamic_smem(kern, max_shared);
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2059,43 +1891,52 @@ int64_t resident_blocks(const void* kern, int smem, int threads = WPB * 32) {
     return (int64_t)std::max(sms, 1) * per_sm;
 }
 
+// The same, looked up once per handle, kernel and size: the attribute and occupancy calls cost about
+// 3 us of host time a launch, which is what bounds a call on a small mesh.
+int64_t launch_plan(pms_elements* h, const void* kern, int smem, int threads, bool max_shared = true) {
+    for (const auto& q : h->plans)
+        if (q.kern == kern && q.smem == smem) return q.resident;
+    const int64_t n = resident_blocks(kern, smem, threads, max_shared);
+    h->plans.push_back({kern, smem, n});
+    return n;
+}
+
 // 2D cells with at most 16 integration points: LPC lanes per cell, 32/LPC cells per warp
+// (h = nullptr: the no-allocation call, which has no handle and takes a block per group of cells)
 template <int NN, int LPC, int UPD, bool DOF, bool DOK, bool CSR>
-void launch_elem2d_lpc(const ElemArgs& a, cudaStream_t st, bool persistent) {
+void launch_elem2d_lpc(pms_elements* h, const ElemArgs& a, cudaStream_t st) {
     constexpr int CPW = 32 / LPC;
     auto kern = element2d_kernel<NN, LPC, UPD, DOF, DOK, CSR>;
     const int smem = smem2_bytes(NN, a.ngauss, CPW, CSR);
-    allow_dynamic_smem((const void*)kern);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     int64_t blocks = ((a.ncell + CPW - 1) / CPW + WPB2 - 1) / WPB2;
-    if (persistent || CSR) blocks = std::min<int64_t>(blocks, resident_blocks((const void*)kern, smem, WPB2 * 32));
+    if (h) blocks = std::min<int64_t>(blocks, launch_plan(h, (const void*)kern, smem, WPB2 * 32));
+    else allow_dynamic_smem((const void*)kern);
     if (CSR) cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), st);
     kern<<<(unsigned)std::max<int64_t>(blocks, 1), WPB2 * 32, smem, st>>>(a);
 }
 
 template <int NN, int UPD, bool DOF, bool DOK, bool CSR>
-void launch_elem2d_t(const ElemArgs& a, cudaStream_t st, bool persistent) {
+void launch_elem2d_t(pms_elements* h, const ElemArgs& a, cudaStream_t st) {
     if constexpr (packed_layout<NN>()) {
         if (a.ngauss <= lanes_packed<NN>()) {
-            launch_elem2d_lpc<NN, lanes_packed<NN>(), UPD, DOF, DOK, CSR>(a, st, persistent);
+            launch_elem2d_lpc<NN, lanes_packed<NN>(), UPD, DOF, DOK, CSR>(h, a, st);
             return;
         }
     }
-    launch_elem2d_lpc<NN, 16, UPD, DOF, DOK, CSR>(a, st, persistent);
+    launch_elem2d_lpc<NN, 16, UPD, DOF, DOK, CSR>(h, a, st);
 }
 
 template <int ND, int NN, int UPD, bool DOF, bool DOK, bool CSR>
 void launch_elem_t(pms_elements* h, const ElemArgs& a) {
     if constexpr (ND == 2 && fits_2d<NN>()) {
         if (a.ngauss <= NG2_MAX) {
-            launch_elem2d_t<NN, UPD, DOF, DOK, CSR>(a, h->stream, true);
+            launch_elem2d_t<NN, UPD, DOF, DOK, CSR>(h, a, h->stream);
             return;
         }
     }
     auto kern = element_kernel<ND, NN, UPD, DOF, DOK, CSR>;
-    allow_dynamic_smem((const void*)kern);
     int64_t blocks = (a.ncell + cells_per_block(NN) - 1) / cells_per_block(NN);
-    blocks = std::min<int64_t>(blocks, resident_blocks((const void*)kern, h->smem_bytes));
+    blocks = std::min<int64_t>(blocks, launch_plan(h, (const void*)kern, h->smem_bytes, WPB * 32));
     if (CSR) cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), h->stream);
     kern<<<(unsigned)blocks, WPB * 32, h->smem_bytes, h->stream>>>(a);
 }
@@ -2209,52 +2050,39 @@ static int64_t value_offset(const pms_elements* h, int64_t A) {
     return h->sym == PMS_SYM_FULL ? (int64_t)h->nd * h->nd * h->pat.bptr[A] : h->tbase[A];
 }
 
-template <int ND, int NN>
-void launch_kk_gather_t(pms_elements* h, double* csr, const int32_t* node_prob, const uint8_t* pmode,
-                        const pms::WorkQueue* q, int64_t node0, int64_t nrows, bool pub) {
-    const bool tri = pub && h->sym != PMS_SYM_FULL;
-    auto kern = tri ? kk_gather_kernel<ND, NN, true> : kk_gather_kernel<ND, NN, false>;
-    if (h->gather_smem > 48 * 1024)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, h->gather_smem);
-    const int64_t np = q ? q->nnode : (nrows >= 0 ? nrows : h->npoint), wpb = h->gather_wpb;
-    const int64_t nw = (np + GatherShape<ND, NN>::G - 1) / GatherShape<ND, NN>::G;  // warps of rows
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nw + wpb - 1) / wpb, 148 * 32));
-    kern<<<blocks, (unsigned)(32 * wpb), h->gather_smem, h->stream>>>(
-        np, h->pat.nbmax, h->d_bptr, h->d_inc_ptr, h->d_inc, h->d_slot, h->d_ke, csr, node_prob, pmode,
-        q ? q->nq : 0, q ? q->node_off : nullptr, q ? q->node_first : nullptr, node0, tri ? h->sym : PMS_SYM_FULL,
-        h->d_kdiag, h->d_tbase);
-}
-
-// CSR gather of the block rows [node0, node0 + nrows) (nrows < 0: all), or of a work queue; pub: into
-// the public layout of the values (pms_elements_set_symmetry), else the full one
-void launch_kk_gather(pms_elements* h, double* csr, const int32_t* node_prob = nullptr,
-                      const uint8_t* pmode = nullptr, const pms::WorkQueue* q = nullptr, int64_t node0 = 0,
-                      int64_t nrows = -1, bool pub = false) {
-    switch (h->kind) {
-    case PMS_TRI3: launch_kk_gather_t<2, 3>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_TRI6: launch_kk_gather_t<2, 6>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_QUA4: launch_kk_gather_t<2, 4>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_QUA8: launch_kk_gather_t<2, 8>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_QUA9: launch_kk_gather_t<2, 9>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_TET4: launch_kk_gather_t<3, 4>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_TET10: launch_kk_gather_t<3, 10>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_HEX8: launch_kk_gather_t<3, 8>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_HEX20: launch_kk_gather_t<3, 20>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_TRI10: launch_kk_gather_t<2, 10>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    case PMS_TRI15: launch_kk_gather_t<2, 15>(h, csr, node_prob, pmode, q, node0, nrows, pub); break;
-    }
+// CSR gather of the block rows [node0, node0 + nrow) into the handle's storage of the values, and
+// their rows of R (ff, nullable)
+void launch_kk_gather(pms_elements* h, double* csr, double* ff, int64_t node0, int64_t nrow) {
+    GatherArgs P;
+    P.node0 = node0;
+    P.nrow = nrow;
+    P.nbmax = h->pat.nbmax;
+    P.bptr = h->d_bptr;
+    P.inc_ptr = h->d_inc_ptr;
+    P.inc = h->d_inc;
+    P.slot = h->d_slot;
+    P.ke = h->d_ke;
+    P.fe = h->d_fe;
+    P.csr = csr;
+    P.ff = ff;
+    P.sym = h->sym;
+    P.kdiag = h->d_kdiag;
+    P.tbase = h->d_tbase;
+    const GatherShape g = gather_shape(h->kind, h->sym != PMS_SYM_FULL, h->pat.nbmax);
+    const int64_t rows = (int64_t)g.rows * g.wpb;
+    const int64_t blocks = std::min<int64_t>((nrow + rows - 1) / rows, launch_plan(h, g.kern, g.smem, 32 * g.wpb, false));
+    void* args[] = {&P};
+    cudaLaunchKernel(g.kern, dim3((unsigned)std::max<int64_t>(blocks, 1)), dim3((unsigned)(32 * g.wpb)), args,
+                     (size_t)g.smem, h->stream);
     h->launches++;
 }
 
-void launch_f_gather(pms_elements* h, double* ff, const pms::WorkQueue* q = nullptr) {
-    const int64_t n = q ? q->nnode : h->npoint;
-    const int nq = q ? q->nq : 0;
-    const int64_t* off = q ? q->node_off : nullptr;
-    const int64_t* first = q ? q->node_first : nullptr;
+void launch_f_gather(pms_elements* h, double* ff) {
+    const int64_t n = h->npoint;
     if (h->nd == 2)
-        f_gather_kernel<2><<<grid_1d(n), 256, 0, h->stream>>>(n, h->d_inc_ptr, h->d_inc, h->d_fe, ff, nq, off, first);
+        f_gather_kernel<2><<<grid_1d(n), 256, 0, h->stream>>>(n, h->d_inc_ptr, h->d_inc, h->d_fe, ff);
     else
-        f_gather_kernel<3><<<grid_1d(n), 256, 0, h->stream>>>(n, h->d_inc_ptr, h->d_inc, h->d_fe, ff, nq, off, first);
+        f_gather_kernel<3><<<grid_1d(n), 256, 0, h->stream>>>(n, h->d_inc_ptr, h->d_inc, h->d_fe, ff);
     h->launches++;
 }
 
@@ -2384,17 +2212,10 @@ int pms_elements_create(const pms_mesh* mesh, const pms_material* materials, int
     }
     h->stream = h->own_stream;
     h->smem_bytes = smem_bytes_for(h->nn, h->nd, h->ng, WPB);
-    {
-        // kk_gather: buffers for G = 32/nnode rows (largest block row each) per warp, up to 8
-        // warps and 48 KB per block
-        const int64_t row_bytes =
-            (int64_t)(h->nn >= 32 ? 1 : 32 / h->nn) * std::max(h->pat.nbmax, 1) * h->nd * h->nd * 8;
-        if (row_bytes > 200 * 1024) {
-            delete h;
-            return PMS_ERR_TOO_LARGE;
-        }
-        h->gather_wpb = (int)std::max<int64_t>(1, std::min<int64_t>(8, (48 * 1024) / row_bytes));
-        h->gather_smem = (int)(h->gather_wpb * row_bytes);
+    // kk_gather: one warp's row buffers (up to 32/nnode rows, each with room for the largest) fit a block
+    if ((int64_t)(32 / h->nn) * std::max(h->pat.nbmax, 1) * h->nd * h->nd * 8 > 200 * 1024) {
+        delete h;
+        return PMS_ERR_TOO_LARGE;
     }
     // the state starts as LocalState::new: zero stress, elastic, zero internal variables
     init_state_kernel<<<grid_1d(h->nip), 256, 0, h->stream>>>(h->nip, h->nc, h->d_mats, h->d_cmat, h->ng, h->d_sig,
@@ -2626,9 +2447,10 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
         h->ev_pending[k].push_back(e);
     };
     if (upd != UPD_NONE || dof || dok) timed(0, [&] { launch_elem(h, a, upd, dof, dok, direct); });
-    if (dof && !direct) timed(1, [&] { launch_f_gather(h, d_ff); });
+    if (dof && !dok && !direct) timed(1, [&] { launch_f_gather(h, d_ff); });
+    double* k_ff = dof ? d_ff : nullptr;  // R comes out of the row gather of K where both are asked for
     if (mem == PMS_MEM_DEVICE || !dok || direct) {
-        if (dok && !direct) timed(2, [&] { launch_kk_gather(h, d_csr, nullptr, nullptr, nullptr, 0, -1, true); });
+        if (dok && !direct) timed(2, [&] { launch_kk_gather(h, d_csr, k_ff, 0, h->npoint); });
         int rc = cuda_check(h);
         if (rc) return rc;
         if (mem == PMS_MEM_HOST) {
@@ -2652,7 +2474,7 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
     timed(2, [&] {
         for (int k = 0; k < NS; k++) {
             const int64_t A0 = h->npoint * k / NS, A1 = h->npoint * (k + 1) / NS;
-            if (A1 > A0) launch_kk_gather(h, d_csr, nullptr, nullptr, nullptr, A0, A1 - A0, true);
+            if (A1 > A0) launch_kk_gather(h, d_csr, k_ff, A0, A1 - A0);
             cudaEventRecord(h->slab_ev[k], h->stream);
             cudaStreamWaitEvent(h->copy_stream, h->slab_ev[k], 0);
             const int64_t v0 = value_offset(h, A0), v1 = value_offset(h, A1);
@@ -2947,8 +2769,6 @@ ElemLaunchShape mode_shape_2d(const ElemArgs& a) {
     constexpr int CPW = 32 / LPC;
     auto kern = element2d_kernel<NN, LPC, UPD_MODE, true, true, true>;
     const int smem = smem2_bytes(NN, a.ngauss, CPW, true);
-    allow_dynamic_smem((const void*)kern);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     int64_t blocks = ((a.ncell + CPW - 1) / CPW + WPB2 - 1) / WPB2;
     blocks = std::min<int64_t>(blocks, resident_blocks((const void*)kern, smem, WPB2 * 32));
     ElemLaunchShape r;
@@ -2969,9 +2789,8 @@ ElemLaunchShape mode_shape(pms_elements* h, const ElemArgs& a) {
         }
     }
     auto kern = element_kernel<ND, NN, UPD_MODE, true, true, true>;
-    allow_dynamic_smem((const void*)kern);
     int64_t blocks = (a.ncell + cells_per_block(NN) - 1) / cells_per_block(NN);
-    blocks = std::min<int64_t>(blocks, resident_blocks((const void*)kern, h->smem_bytes));
+    blocks = std::min<int64_t>(blocks, resident_blocks((const void*)kern, h->smem_bytes, WPB * 32));
     ElemLaunchShape r;
     r.func = (const void*)kern;
     r.grid = (unsigned)std::max<int64_t>(blocks, 1);
@@ -3090,7 +2909,7 @@ template <int ND, int NN, bool DOF, bool DOK>
 void noalloc_launch_t(const ElemArgs& a, int smem, cudaStream_t st) {
     if constexpr (ND == 2 && fits_2d<NN>()) {
         if (a.ngauss <= NG2_MAX) {
-            launch_elem2d_t<NN, UPD_NONE, DOF, DOK, false>(a, st, false);
+            launch_elem2d_t<NN, UPD_NONE, DOF, DOK, false>(nullptr, a, st);
             return;
         }
     }

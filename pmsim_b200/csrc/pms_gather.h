@@ -1,0 +1,49 @@
+// pms_gather.h -- row gather of the element matrices into the CSR values of K and into R
+// (pms_gather.cu), and the layout of the element matrices it reads.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace pms {
+
+// Number of node-pair blocks (a', b'), a' <= b', before block (a, b) of the upper layout.
+__host__ __device__ constexpr int upper_block(int nn, int a, int b) { return a * nn - a * (a - 1) / 2 + (b - a); }
+// Upper layout of an element matrix: entry (i, j) of block (a, b), a <= b, at
+// BB*upper_block(a, b) + i*ND + j.  A block's entries are contiguous, so the row gather reads block
+// (a, b) and the transpose of block (b, a) alike: whole runs of blocks on the one side, 72 (32 in 2D)
+// contiguous bytes on the other.
+template <int NN, int ND>
+__host__ __device__ constexpr int upper_entry(int a, int b, int i, int j) {
+    return ND * ND * upper_block(NN, a, b) + i * ND + j;
+}
+
+struct GatherArgs {
+    int64_t node0, nrow;  // block rows [node0, node0 + nrow)
+    int nbmax;            // largest block row
+    const int64_t* bptr;
+    const int64_t* inc_ptr;
+    const int32_t* inc;   // incidences of a node, ascending cells: cell*nn + local node
+    const int16_t* slot;  // [k*nn + b]: column slot of local node b of incidence k in the block row
+    const double* ke;     // [cell][upper layout]
+    const double* fe;     // [cell][node][ND]
+    double* csr;
+    double* ff;  // nullable: no R
+    // triangle storages (sym = PMS_SYM_LOWER: columns <= row, PMS_SYM_UPPER: columns >= row;
+    // src/base/assembly.rs:92-122): the other entries are not written out, and row (A, i) starts at
+    // tbase[A] plus the lengths of rows (A, 0..i-1); kdiag[A] = A's own position in its block row
+    int sym;
+    const int32_t* kdiag;
+    const int64_t* tbase;
+};
+
+// Kernel and launch shape of an element kind's gather.
+struct GatherShape {
+    const void* kern;
+    int rows;  // block rows per warp
+    int wpb;   // warps per block
+    int smem;  // bytes per block
+};
+GatherShape gather_shape(int kind, bool triangle, int nbmax);
+
+}  // namespace pms
