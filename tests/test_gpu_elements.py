@@ -289,3 +289,54 @@ def test_bhatti_1d6_plane_stress_on_device():
     out = {}
     sol.solve(lambda step, t, u, e: out.setdefault("u", u.copy()))
     np.testing.assert_allclose(out["u"], pb["golden"]["uu_correct"], rtol=0, atol=1e-14)
+
+
+@pytest.mark.parametrize("kind,ngauss,n", [(M.HEX8, 8, (1, 1, 1)), (M.HEX8, 8, (2, 1, 1)), (M.HEX8, 8, (7, 1, 1)),
+                                           (M.HEX8, 1, (5, 2, 1)), (M.HEX8, 27, (5, 2, 1)), (M.HEX8, 8, (18, 18, 17)),
+                                           (M.TET4, 1, (1, 1, 1)), (M.TET4, 4, (1, 1, 1)), (M.TET4, 4, (3, 1, 3)),
+                                           (M.TET4, 4, (13, 12, 16))])
+def test_cells_packed_into_warps(kind, ngauss, n):
+    """Hex8 and Tet4 run three and eight cells to a warp: one cell, ragged last groups, more groups than
+    the device holds at once, and the rules that fit the slots and that do not, against the oracle at the
+    parity tolerance (the separate calls too)."""
+    from pmsim_b200.elements import Elements, Material
+    m = perturbed_mesh(kind, seed=3, n=n)
+    g = Elements(m, Material.von_mises(E, NU, H, Z0), ngauss=ngauss)
+    o = oracle.OracleElements(m, 1, oracle.Params(E, NU, H, Z0), ngauss=ngauss, sym_tol=-1.0, nthreads=0)
+    indptr, indices = g.csr_pattern()
+    ddu = plastic_ddu(m, seed=4)
+    g.initialize_internal_values()
+    o.initialize()
+    g.backup_secondary_values()
+    ff, kv = np.zeros(g.ndof), np.zeros(g.nnz)
+    g.update_and_assemble(ddu, ff, kv)
+    o.update_secondary_values(ddu)
+    sig, ivs, el = g.get_state()
+    assert np.array_equal(el, o.elastic)
+    assert_close(sig, o.sig, what="sigma")
+    assert_close(ivs, o.ivs, what="[z, lambda]")
+    fo, ko = o.assemble_f_int(), oracle_csr_values(o, indptr, indices)
+    assert_close(ff, fo, what="f_int")
+    assert_close(kv, ko, what="K")
+    assert_close(g.assemble_f_int(), fo, what="f_int alone")
+    assert_close(g.assemble_kk(), ko, what="K alone")
+
+
+@pytest.mark.parametrize("kind", [M.QUA8, M.TRI3, M.HEX8], ids=["qua8", "tri3", "hex8"])
+def test_values_that_start_on_an_odd_eight_bytes(kind):
+    """The CSR values may start anywhere a double may: the same bits as at a 16-byte boundary."""
+    import torch
+    m, g, _ = make(kind, seed=6)
+    g.initialize_internal_values()
+    g.backup_secondary_values()
+    ddu = torch.tensor(plastic_ddu(m, seed=7), device="cuda")
+    out = []
+    for shift in (0, 1):
+        ff = torch.zeros(g.ndof, dtype=torch.float64, device="cuda")
+        kv = torch.zeros(g.nnz + 2, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        g.update_and_assemble(ddu, ff, kv[shift:shift + g.nnz])
+        g.sync()
+        out.append((ff.cpu().numpy(), kv[shift:shift + g.nnz].cpu().numpy()))
+        assert float(kv[:shift].abs().sum()) == 0.0 and float(kv[shift + g.nnz:].abs().sum()) == 0.0
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
