@@ -922,6 +922,9 @@ struct pms_batch {
     cudaEvent_t ev_fork = nullptr, ev_cls[5] = {};
     int cls_off[6] = {};
     int team_cmax = 8;
+    bool fit_teams = true;         // team sizes follow the load (until a tuning is set)
+    int budget_factor = 1;         // PCG budget of a tick, in units of the tuned one
+    int team_slots[5] = {};        // teams of 1, 2, 4, 8, 16 CTAs that the device holds at once
     cudaGraphExec_t graph = nullptr;
     int graph_iters_captured = 0;
     std::string last_error;
@@ -1206,15 +1209,80 @@ int pcg_phase(pms_batch* b, int nteam, int nwide, int budget, bool exact) {
     return PMS_OK;
 }
 
+// Teams of each size that the device holds at once, for the launch shape of the current tuning.
+void count_team_slots(pms_batch* b) {
+    const bool two = tpr_of(b->v.nd) == 8;
+    const void* kern = nullptr;
+    switch (b->tune.team_threads) {
+        case 256: kern = two ? (const void*)pcg_team_kernel<256, 8> : (const void*)pcg_team_kernel<256, 16>; break;
+        case 1024: kern = two ? (const void*)pcg_team_kernel<1024, 8> : (const void*)pcg_team_kernel<1024, 16>; break;
+        default: kern = two ? (const void*)pcg_team_kernel<512, 8> : (const void*)pcg_team_kernel<512, 16>; break;
+    }
+    for (int c = 0; c < NCLASS; c++) {
+        b->team_slots[c] = 0;
+        if ((1 << c) > b->team_cmax) continue;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1u << c);
+        cfg.blockDim = dim3((unsigned)b->tune.team_threads);
+        cfg.dynamicSmemBytes = team_smem_bytes(b->v.nd, b->tune.team_threads);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1u << c;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&b->team_slots[c], kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            b->team_slots[c] = 0;
+        }
+    }
+}
+
+// Team size (as its power of two) of a problem of nch chunks at `per` chunks per CTA; -1: too large.
+int team_class(const pms_batch* b, int64_t nch, int per) {
+    for (int c = 0; (1 << c) <= b->team_cmax; c++)
+        if ((nch + (1 << c) - 1) >> c <= per) return c;
+    return -1;
+}
+
 // Team lists of the problems selected by `want` (grouped by team size) and the count of
-// batch-wide ones.
+// batch-wide ones.  Without a tuning of the caller's the teams follow the load: the fewest chunks per CTA
+// at which all of them are resident at once.  A team CTA fills an SM, so 32 footings of 2 to 13
+// chunks at one chunk per CTA take 3.5 waves of 7 us an iteration, at two chunks one wave of 9 us; as problems
+// finish, the others' teams grow.  (One load step of those footings: 45 ms at one chunk, 34 at two,
+// 44 at four.)  While the device is full the ticks are four times as long: a tick's host work costs about
+// 0.2 ms (128 iterations a tick 34 ms, 512 30 ms).  The iterates depend on neither.
 void build_lists(pms_batch* b, const std::vector<uint8_t>& want, int& nteam, int& nwide) {
     b->h_list.clear();
     nwide = 0;
+    int per = 0;
+    b->budget_factor = 1;
+    if (b->fit_teams) {
+        const int cap = team_node_capacity(b->v.nd, b->tune.team_threads) / CHN;
+        for (per = std::max(1, b->tune.team_chunks); per < cap; per++) {
+            double load = 0.0;
+            for (int p = 0; p < b->np; p++) {
+                if (!want[p] || b->engine[p] == 0) continue;
+                const int c = team_class(b, b->pnch[p], per);
+                load += c < 0 || b->team_slots[c] < 1 ? 1e9 : 1.0 / b->team_slots[c];
+            }
+            if (load <= 1.0) break;
+        }
+        if (per > std::max(1, b->tune.team_chunks)) b->budget_factor = 4;
+    }
+    std::vector<int8_t> cls(b->np, -1);
+    for (int p = 0; p < b->np; p++) {
+        if (!want[p] || b->engine[p] == 0) continue;
+        if (per > 0) cls[p] = (int8_t)team_class(b, b->pnch[p], per);
+        if (cls[p] < 0)  // as tuned
+            for (int c = 0; c < NCLASS; c++)
+                if (b->engine[p] == (1 << c)) cls[p] = (int8_t)c;
+    }
     for (int c = 0; c < NCLASS; c++) {
         b->cls_off[c] = (int)b->h_list.size();
         for (int p = 0; p < b->np; p++)
-            if (want[p] && b->engine[p] == (1 << c)) b->h_list.push_back(p);
+            if (cls[p] == c) b->h_list.push_back(p);
     }
     b->cls_off[NCLASS] = (int)b->h_list.size();
     for (int p = 0; p < b->np; p++)
@@ -1382,6 +1450,7 @@ int pms_batch_create(pms_elements* el, int32_t nproblem, const int64_t* point_pt
     b->it.assign(nproblem, 0);
     b->pnch.assign(nproblem, 0);
     for (int p = 0; p < nproblem; p++) b->pnch[p] = pchunk[p + 1] - pchunk[p];
+    count_team_slots(b);
     if (assign_engines(b) || cudaDeviceSynchronize() != cudaSuccess) {
         delete b;
         return PMS_ERR_CUDA;
@@ -1507,7 +1576,7 @@ int pms_batch_tick(pms_batch* b, const uint8_t* cmd, const double* c_values, int
     int nteam = 0, nwide = 0;
     build_lists(b, b->solving, nteam, nwide);
     if (nteam + nwide > 0) {
-        rc = pcg_phase(b, nteam, nwide, std::max(1, b->tune.pcg_budget), false);
+        rc = pcg_phase(b, nteam, nwide, std::max(1, b->tune.pcg_budget) * b->budget_factor, false);
         if (rc) return rc;
         std::vector<uint8_t> wa(np), ca(np);
         cudaMemcpyAsync(wa.data(), b->d_pcg_active, np, cudaMemcpyDeviceToHost, st);
@@ -1813,6 +1882,7 @@ int pms_batch_set_tuning(pms_batch* b, const pms_batch_tuning* t) {
     for (int p = 0; p < b->np; p++)
         if (b->solving[p]) return bfail(b, PMS_ERR_INVALID, "tuning cannot change while a linear solve is under way");
     b->tune = *t;
+    b->fit_teams = false;
     if (cudaStreamSynchronize(b->v.stream) != cudaSuccess) return PMS_ERR_CUDA;
     return assign_engines(b);
 }
@@ -1882,6 +1952,7 @@ int time_candidate(pms_batch* b, const pms_batch_tuning& cand, int iters, float*
 int pms_batch_time_pcg(pms_batch* b, const pms_batch_tuning* t, int32_t iterations, double* ms) {
     if (!b || !t || !ms || iterations < 1) return PMS_ERR_INVALID;
     const pms_batch_tuning keep = b->tune;
+    const bool fit = b->fit_teams;
     int rc = pms_batch_set_tuning(b, t);
     if (rc) return rc;
     rc = timing_setup(b);
@@ -1889,6 +1960,7 @@ int pms_batch_time_pcg(pms_batch* b, const pms_batch_tuning* t, int32_t iteratio
     if (!rc) rc = time_candidate(b, *t, iterations, &m);
     *ms = m;
     b->tune = keep;
+    b->fit_teams = fit;
     int rc2 = assign_engines(b);
     int rc3 = pms_batch_reset(b);
     return rc ? rc : (rc2 ? rc2 : rc3);
@@ -1904,6 +1976,8 @@ int pms_batch_autotune(pms_batch* b, pms_batch_tuning* out) {
     int64_t maxdof = 0;
     for (int p = 0; p < np; p++) maxdof = std::max(maxdof, b->pndof[p]);
     const pms_batch_tuning keep = b->tune;
+    const bool fit = b->fit_teams;
+    b->fit_teams = false;  // the candidates are timed, and the best one runs, as they are
     std::vector<pms_batch_tuning> cands;
     {
         pms_batch_tuning c = keep;
@@ -1933,6 +2007,7 @@ int pms_batch_autotune(pms_batch* b, pms_batch_tuning* out) {
         }
     }
     b->tune = rc ? keep : best;
+    if (rc) b->fit_teams = fit;
     int rc2 = assign_engines(b);
     int rc3 = pms_batch_reset(b);
     if (!rc && out) *out = b->tune;

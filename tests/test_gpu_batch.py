@@ -253,3 +253,20 @@ def test_batch_constant_tangent_matches_oracle(name):
     for a, b in zip(runs[False], runs[True]):
         assert np.array_equal(a, b)
     assert sum(len(h) for h in osol.history) > pb["nsteps"] * 2  # modified Newton takes extra iterations
+
+
+def test_team_sizes_that_follow_the_load_give_the_same_bits():
+    """Without a tuning the PCG teams take as few CTAs per problem as lets all of them run at once, and
+    grow as problems finish; a tuning fixes them.  A batch that fills the device several times over
+    and one that does not: the same iterates either way."""
+    from pmsim_b200.batch import BatchSolver
+    rng = np.random.default_rng(23)
+    for count in (3, 60):
+        probs = [footing(int(rng.integers(8, 22)), int(rng.integers(4, 12)), float(1e4 * np.exp(rng.normal(0, 0.3))),
+                         float(rng.uniform(8, 20)), float(rng.uniform(0.5, 2.0)), nsteps=1) for _ in range(count)]
+        a, b = BatchSolver(probs), BatchSolver(probs)
+        b.set_tuning(**b.tuning())
+        ra, rb = a.solve_step(), b.solve_step()
+        for x, y in zip(ra, rb):
+            assert np.array_equal(x, y)
+        assert np.array_equal(a.u(), b.u())
