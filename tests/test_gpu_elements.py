@@ -340,3 +340,28 @@ def test_values_that_start_on_an_odd_eight_bytes(kind):
         out.append((ff.cpu().numpy(), kv[shift:shift + g.nnz].cpu().numpy()))
         assert float(kv[:shift].abs().sum()) == 0.0 and float(kv[shift + g.nnz:].abs().sum()) == 0.0
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("kind,n", [(M.QUA8, (20, 21, 1)), (M.QUA8, (60, 40, 1)), (M.HEX20, (7, 6, 5))],
+                         ids=["below one piece", "about one piece", "several pieces"])
+def test_host_arrays_pageable_pinned_and_device(kind, n):
+    """K into pageable memory (in pinned pieces of 262,144 values once it is that large), into pinned
+    memory and on the device: the same bits, for both triangles' storage and one's."""
+    import torch
+    m = perturbed_mesh(kind, seed=2, n=n)
+    from pmsim_b200.elements import Elements, Material
+    g = Elements(m, Material.von_mises(E, NU, H, Z0))
+    g.initialize_internal_values()
+    g.backup_secondary_values()
+    ddu = plastic_ddu(m, seed=3)
+    for sym in ("full", "lower"):
+        g.set_symmetry(sym)
+        d_kv = torch.zeros(g.nnz, dtype=torch.float64, device="cuda")
+        d_ff = torch.zeros(g.ndof, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        g.update_and_assemble(torch.tensor(ddu, device="cuda"), d_ff, d_kv)
+        g.sync()
+        for kv in (np.zeros(g.nnz), torch.zeros(g.nnz, dtype=torch.float64).pin_memory().numpy()):
+            ff = np.zeros(g.ndof)
+            g.update_and_assemble(ddu, ff, kv)
+            assert np.array_equal(kv, d_kv.cpu().numpy()) and np.array_equal(ff, d_ff.cpu().numpy())
