@@ -284,8 +284,8 @@ int pms_batch_tick(pms_batch* b, const uint8_t* cmd, const double* c_values, int
 /* The same lock-step load step as pms_batch_solve_step (same arguments, same results bit for bit),
  * with the Newton loop resident on the device: one CUDA graph launch per load step, in which a
  * conditional WHILE node runs every active problem's Newton iterations -- element pass, residual
- * test, PCG start, a nested WHILE over PCG iterations, completion and update -- with the
- * per-problem sequencing of SolverImplicit::iterate (src/fem/solver_implicit.rs:187-272) done by
+ * test, PCG start, the PCG of every problem (one cooperative kernel, or for batches of many nodes a
+ * nested WHILE over iterations), completion and update -- with the per-problem sequencing of SolverImplicit::iterate (src/fem/solver_implicit.rs:187-272) done by
  * controller kernels; the host waits once per load step.  Every problem's PCG runs on the
  * batch-wide engine (the engines give the same bits).  The graph is built on the first call and
  * kept by the batch.  Not while a tick-driven linear solve is under way (PMS_ERR_INVALID). */
@@ -298,8 +298,12 @@ int64_t pms_batch_host_syncs(const pms_batch* b);
  * A problem with at most team_max_ndof DOFs runs its whole PCG on a thread-block cluster ("team")
  * of C = 1, 2, 4, 8 or 16 CTAs of team_threads threads (256, 512 or 1024), its vectors resident in
  * the CTAs' shared memory; C is the smallest team whose CTAs hold at most team_chunks 128-node
- * chunks each (0: as many as fit).  Other problems run the batch-wide kernels, graph_iters
- * iterations per CUDA-graph launch.  pcg_budget bounds the PCG iterations a problem gets per tick.
+ * chunks each (0: as many as fit).  Until pms_batch_set_tuning or pms_batch_autotune is called the teams
+ * follow the load instead: no smaller chunks per CTA than team_chunks, but as many as it takes for all
+ * teams to be resident at once, and longer ticks while they fill the device.  Other problems run the
+ * batch-wide kernels, graph_iters iterations per CUDA-graph launch (eight times as many per launch
+ * of the cooperative kernel that batches of few nodes take).  pcg_budget bounds the PCG iterations a
+ * problem gets per tick.
  * No counterpart in the reference (its solve is a direct factorisation,
  * src/fem/linear_system.rs:185-201). */
 typedef struct pms_batch_tuning {

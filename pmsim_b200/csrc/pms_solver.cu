@@ -20,8 +20,9 @@
 // Two PCG engines, one arithmetic.  A problem whose vectors fit the shared memory of up to 16 CTAs
 // runs its whole PCG loop on a thread-block cluster (pcg_team_kernel: distributed shared memory,
 // hardware cluster barriers, every problem at its own pace, resumable across ticks); larger
-// problems run the batch-wide kernels (spmv+dot, update, beta+direction), captured in a CUDA graph.  Both engines call the same per-node and per-row functions and reduce
-// through the same trees: 128-node chunks that never straddle two problems, each summed by the
+// problems run the batch-wide engine: one cooperative kernel with grid barriers for batches of few
+// nodes, else three kernels an iteration (spmv+dot, update, beta+direction) in a CUDA graph.  All of them
+// call the same per-node and per-row functions and reduce through the same trees: 128-node chunks that never straddle two problems, each summed by the
 // fixed pairing (t, t+s), s = 64..1, and a problem's chunk partials summed in chunk order.  A
 // problem's iterates are therefore bit-identical whichever engine runs it and whichever problems
 // share the batch, so the engine threshold and launch shapes (chosen by pms_batch_autotune) change
@@ -393,7 +394,7 @@ pcg_init_scalars_kernel(int np, const uint8_t* active, const uint8_t* engine, co
     cta_active[p] = engine[p] ? go : 0;
 }
 
-// ---- batch-wide PCG engine (one CUDA graph node per kernel) --------------------------------
+// ---- batch-wide PCG engine, many nodes: three kernels an iteration, one CUDA graph node each ----
 
 // q = K p on the nodes of one chunk quarter (32 nodes, one group of TPR lanes each, node_rows_dot),
 // then the quarter's partial of p.q by the warp tree.  Block b covers quarter b % 4 of chunk b / 4.
@@ -503,6 +504,375 @@ pcg_beta_direction_kernel(SolverArgs S, int par, const double* part_rz, const do
             const int64_t i = node * S.nd + d;
             dof_direction(S.pres_idx[i], beta, z + i, p + i);
         }
+    }
+}
+
+// ---- batch-wide PCG engine, up to WIDE_MAX_CHUNKS chunks: one cooperative kernel ---------------------
+// One cooperative launch runs up to `budget` iterations of every problem it finds active.  The blocks own
+// chunk quarters (32 nodes) of the active problems, spread evenly and dealt again every few
+// iterations as problems finish; the vectors stay in global memory (L2), and two grid barriers order an
+// iteration:
+//   A  q = K p on the own quarters, with p = z + beta p' formed on the way (gathered from z and the last p';
+//      the owner also stores p), partials of p.q
+//   -- barrier -- alpha from the partials (every block of a problem sums the same ones in the same order)
+//   B  x, r, z of the own quarters, partials of r.z and r.r
+//   -- barrier -- beta, iteration count and stopping test from the partials
+// Bound by the barriers (2.3 to 3 us each, L2 round trips) and the dependent loads of a phase.  Time of an
+// iteration, three kernels in a CUDA graph and this: 661 nodes (20x10 Qua8) 13.9 and 10.3 us, 1,331 (10x10x10 Hex8)
+// 14.1 and 10.9, 9,261 (20^3) 14.6 and 13.4, six footings of 13,236 14.9 and 14.1; but 15,425 15.0 and 17.4,
+// 29,791 26.1 and 26.6, 1,075,133 239 and 304: beyond WIDE_MAX_CHUNKS, where blocks come and go with the work and hide
+// each other's latencies, the graph stays.
+//
+// The per-problem scalars are double-buffered by iteration parity (an iteration reads one and writes the
+// other), so no block reads what another writes in the same phase; a launch ends with buffer 0 current.
+constexpr int64_t WIDE_MAX_CHUNKS = 104;   // 13,312 nodes
+constexpr int WIDE_THREADS = 512;
+constexpr int WIDE_DEAL = 32;              // iterations between two deals of the quarters (even)
+constexpr int WIDE_SPIN_LIMIT = 1 << 23;   // polls of a grid barrier (seconds; a phase takes microseconds)
+
+struct WideQuarter {  // 32 nodes of one problem
+    int64_t node0, bb;  // first node, its first block
+    int32_t part, nn;   // place of the partials, nodes
+    int32_t rel[33];    // blocks before each node
+    int32_t pad;
+};
+
+struct WideArgs {
+    const WideQuarter* quarter;  // four per chunk
+    const int32_t* bcol;
+    const double* val;
+    const double* binv;
+    double *p0, *p1;  // the direction by iteration parity; p0 is current between launches
+    double *q, *x, *r, *z;
+    double *part_pq, *part_rz, *part_rr;  // four per chunk
+    double* rho;                          // [2][np]
+    const double* r0;
+    int32_t* iters;        // [2][np]
+    unsigned* ctl;         // zero at launch: barrier arrivals, problems finished in this launch, failure flag
+    double rtol;
+    int32_t max_iter;
+    int32_t budget;        // iterations (even)
+    int32_t stop;          // end, at an even iteration, once this many problems have finished
+};
+
+// What a block holds of its share in shared memory: runs of quarters of one problem each (with the problem's
+// scalars), and the first WIDE_DESC quarters.
+struct WideRun {
+    int64_t c0, c1;  // chunks of the problem
+    double rho, r0;
+    int32_t prob, iters, off, len;  // its first quarter (of the problem) and count here
+    int32_t first;                  // its first quarter here
+    int32_t active;
+};
+constexpr int WIDE_KEEP = 16;  // quarters whose p and q stay in shared memory between the phases
+constexpr int WIDE_DESC = 64;
+__host__ __device__ inline size_t wide_smem_bytes(int nd, int nruns, int share) {
+    return (size_t)(share < WIDE_KEEP ? share : WIDE_KEEP) * 64 * nd * 8 + (size_t)nruns * sizeof(WideRun) +
+           (size_t)(share < WIDE_DESC ? share : WIDE_DESC) * sizeof(WideQuarter);
+}
+
+// The quarters of every problem, four per chunk (one warp each).
+__global__ void wide_quarters_kernel(int64_t nquarter, const int64_t* chunk_node0, const int32_t* chunk_nnode,
+                                     const int64_t* bptr, WideQuarter* out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t Q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (Q >= nquarter) return;
+    const int64_t ch = Q >> 2;
+    const int k = (int)(Q & 3), nn = max(0, min(32, chunk_nnode[ch] - 32 * k));
+    const int64_t node0 = chunk_node0[ch] + (nn > 0 ? 32 * k : 0), bb = bptr[node0];
+    WideQuarter& w = out[Q];
+    if (lane == 0) {
+        w.node0 = node0;
+        w.bb = bb;
+        w.part = (int32_t)Q;
+        w.nn = nn;
+    }
+    for (int m = lane; m <= nn; m += 32) w.rel[m] = (int32_t)(bptr[node0 + m] - bb);
+}
+
+template <int TPR>
+__global__ void __launch_bounds__(WIDE_THREADS, 2) pcg_wide_kernel(SolverArgs S, WideArgs W, int maxruns, int maxshare) {
+    constexpr int ND = TPR == 8 ? 2 : 3;              // the lanes per node follow the dimension
+    constexpr int QT = 32 * TPR, QPP = WIDE_THREADS / QT;  // threads per quarter, quarters at a time
+    constexpr int NW = WIDE_THREADS / 32;
+    extern __shared__ __align__(16) double wide_smem[];
+    double* pq_own = wide_smem;  // [quarter][p, q][32*ND]
+    WideRun* runs = reinterpret_cast<WideRun*>(wide_smem + min(maxshare, WIDE_KEEP) * 64 * ND);
+    WideQuarter* desc = reinterpret_cast<WideQuarter*>(runs + maxruns);
+    // quarter t of a run
+    auto quarter = [&](const WideRun& r, int t) -> const WideQuarter& {
+        return r.first + t < WIDE_DESC ? desc[r.first + t] : W.quarter[4 * r.c0 + r.off + t];
+    };
+    __shared__ double sh[8];
+    __shared__ double qs[QPP * 32 * ND];
+    __shared__ unsigned wsum[2 * NW];
+    __shared__ int nruns_s;
+    __shared__ bool failed_s;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned G = gridDim.x;
+    unsigned target = 0;
+    volatile unsigned* ctl = W.ctl;
+
+    // every block arrives, then waits for all (false: a wait ran out, here or elsewhere)
+    auto barrier = [&]() -> bool {
+        __syncthreads();
+        target += G;
+        if (tid == 0) {
+            __threadfence();
+            atomicAdd(W.ctl, 1u);
+            for (int n = 0; (int)(ctl[0] - target) < 0; n++)
+                if (n >= WIDE_SPIN_LIMIT || ((n & 63) == 63 && ctl[2] != 0)) {
+                    atomicExch(W.ctl + 2, 1u);
+                    break;
+                }
+            __threadfence();
+            failed_s = ctl[2] != 0;
+        }
+        __syncthreads();
+        return !failed_s;
+    };
+    // quarters of a problem's total, into s4 (as problem_total: 128 threads add the chunks t, t + 128, ...)
+    auto total = [&](const double* part4, int64_t c0, int64_t c1, double* s4, int t) {
+        double v = 0.0;
+        for (int64_t c = c0 + t; c < c1; c += CHN)
+            v += quarters<false>(part4[4 * c], part4[4 * c + 1], part4[4 * c + 2], part4[4 * c + 3]);
+        v = warp_tree<false>(v);
+        if ((t & 31) == 0) s4[t >> 5] = v;
+    };
+    // deals the quarters of the problems that `present` names: this block's share, with the scalars of parity
+    // `par`; returns the number of problems
+    auto deal = [&](auto present, int par) -> int {
+        const int np = S.np;
+        const int p0 = (int)((int64_t)tid * np / WIDE_THREADS), p1 = (int)((int64_t)(tid + 1) * np / WIDE_THREADS);
+        unsigned len = 0, cnt = 0;
+        for (int p = p0; p < p1; p++)
+            if (present(p)) {
+                len += 4u * (unsigned)(S.pchunk[p + 1] - S.pchunk[p]);
+                cnt++;
+            }
+        unsigned incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += v;
+        }
+        cnt = __reduce_add_sync(FULL, cnt);
+        __syncthreads();  // the last use of what follows
+        if (lane == 31) wsum[wid] = incl;
+        if (lane == 0) wsum[NW + wid] = cnt;
+        if (tid == 0) nruns_s = 0;
+        __syncthreads();
+        unsigned before = 0, all = 0, n = 0;
+        for (int k = 0; k < NW; k++) {
+            before += k < wid ? wsum[k] : 0;
+            all += wsum[k];
+            n += wsum[NW + k];
+        }
+        const unsigned lo = (unsigned)((uint64_t)blockIdx.x * all / G), hi = (unsigned)((uint64_t)(blockIdx.x + 1) * all / G);
+        unsigned start = before + incl - len;
+        for (int p = p0; p < p1 && start < hi; p++)
+            if (present(p)) {
+                const unsigned l = 4u * (unsigned)(S.pchunk[p + 1] - S.pchunk[p]);
+                const unsigned a = max(lo, start), e = min(hi, start + l);
+                if (a < e) {
+                    WideRun& r = runs[atomicAdd(&nruns_s, 1)];
+                    r.prob = p;
+                    r.off = (int32_t)(a - start);
+                    r.len = (int32_t)(e - a);
+                    r.first = (int32_t)(a - lo);
+                    r.c0 = S.pchunk[p];
+                    r.c1 = S.pchunk[p + 1];
+                    r.rho = W.rho[par * np + p];
+                    r.r0 = W.r0[p];
+                    r.iters = W.iters[par * np + p];
+                    r.active = S.pcg_active[par * np + p];
+                }
+                start += l;
+            }
+        __syncthreads();
+        for (int rn = 0; rn < nruns_s; rn++) {
+            const WideRun& r = runs[rn];
+            for (int t = wid; t < r.len && r.first + t < WIDE_DESC; t += NW) {  // one warp per quarter
+                const int32_t* src = reinterpret_cast<const int32_t*>(W.quarter + 4 * r.c0 + r.off + t);
+                int32_t* dst = reinterpret_cast<int32_t*>(desc + r.first + t);
+                for (int m = lane; m < (int)(sizeof(WideQuarter) / 4); m += 32) dst[m] = src[m];
+            }
+        }
+        __syncthreads();
+        return (int)n;
+    };
+
+    if (blockIdx.x == 0)  // buffer 1 of the activity flags names nobody that buffer 0 does not
+        for (int p = tid; p < S.np; p += WIDE_THREADS)
+            if (!S.pcg_active[p]) S.pcg_active[S.np + p] = 0;
+    const int nactive = deal([&](int p) { return S.pcg_active[p] != 0; }, 0);
+    if (nactive == 0) return;
+
+    for (int it = 0;; it++) {
+        const int s = it & 1;  // parity of the scalars after phase C of this iteration, and of its direction
+        double* pn = s ? W.p1 : W.p0;
+        const double* po = s ? W.p0 : W.p1;
+        const int nruns = nruns_s;
+        for (int rn = 0; rn < nruns; rn++) {
+            WideRun& run = runs[rn];
+            const int pr = run.prob, len = run.len, first = run.first;
+            double beta = 0.0;
+            if (it > 0) {
+                const bool lead = run.off == 0 && tid == 0;
+                const int nxt = s * S.np + pr;
+                if (!run.active) {  // finished at an earlier iteration
+                    if (lead) {
+                        S.pcg_active[nxt] = 0;
+                        W.rho[nxt] = run.rho;
+                        W.iters[nxt] = run.iters;
+                    }
+                    continue;
+                }
+                if (tid < CHN) total(W.part_rz, run.c0, run.c1, sh, tid);
+                else if (tid < 2 * CHN) total(W.part_rr, run.c0, run.c1, sh + 4, tid - CHN);
+                __syncthreads();
+                const double a = quarters<false>(sh[0], sh[1], sh[2], sh[3]);
+                const double b = quarters<false>(sh[4], sh[5], sh[6], sh[7]);
+                double rh = run.rho;
+                int32_t n = run.iters;
+                const bool done = pcg_scalar_step(a, b, rh, run.r0, n, W.rtol, W.max_iter, beta);
+                __syncthreads();  // sh and the run are read
+                if (tid == 0) {
+                    run.rho = rh;
+                    run.iters = n;
+                    run.active = done ? 0 : 1;
+                }
+                if (lead) {
+                    W.rho[nxt] = rh;
+                    W.iters[nxt] = n;
+                    S.pcg_active[nxt] = done ? 0 : 1;
+                    if (done) atomicAdd(W.ctl + 1, 1u);
+                }
+                if (done) continue;
+                if (it >= W.budget) {  // leave the next direction in buffer 0
+                    for (int t = wid; t < len; t += NW) {
+                        const WideQuarter& w = quarter(run, t);
+                        if (lane < w.nn) {
+                            const int64_t i0 = (w.node0 + lane) * ND;
+#pragma unroll
+                            for (int d = 0; d < ND; d++)
+                                W.p0[i0 + d] = S.pres_idx[i0 + d] >= 0 ? 0.0 : fma(beta, po[i0 + d], W.z[i0 + d]);
+                        }
+                    }
+                    continue;
+                }
+            }
+            // ---- A: q = K p
+            const int g = tid / QT, grp = (tid % QT) / TPR, sub = tid % TPR;
+            for (int t0 = 0; t0 < len; t0 += QPP) {
+                const bool have = t0 + g < len;
+                const WideQuarter& w = quarter(run, have ? t0 + g : 0);
+                const int nn = have ? w.nn : 0;
+                const bool on = grp < nn;
+                const int64_t bb = on ? w.bb + w.rel[grp] : 0;
+                const int nba = on ? w.rel[grp + 1] - w.rel[grp] : 0;
+                const int64_t A = w.node0 + grp;
+                double sv[ND];
+                if (it == 0)
+                    node_rows_dot<ND, TPR>(bb, nba, sub, W.val, W.bcol,
+                                           [&](int32_t c, double (&x)[ND]) {
+#pragma unroll
+                                               for (int j = 0; j < ND; j++) x[j] = pn[(int64_t)c * ND + j];
+                                           },
+                                           sv);
+                else  // (prescribed DOFs: z = 0 and p' = 0, so p = 0 as stored)
+                    node_rows_dot<ND, TPR>(bb, nba, sub, W.val, W.bcol,
+                                           [&](int32_t c, double (&x)[ND]) {
+#pragma unroll
+                                               for (int j = 0; j < ND; j++)
+                                                   x[j] = fma(beta, po[(int64_t)c * ND + j], W.z[(int64_t)c * ND + j]);
+                                           },
+                                           sv);
+                const int keep = first + t0 + g;
+                if (on && sub == 0) {
+#pragma unroll
+                    for (int i = 0; i < ND; i++) {
+                        const double v = S.pres_idx[A * ND + i] >= 0 ? 0.0 : sv[i];
+                        qs[(g * 32 + grp) * ND + i] = v;
+                        if (keep < WIDE_KEEP) pq_own[(2 * keep + 1) * 32 * ND + grp * ND + i] = v;
+                        else W.q[A * ND + i] = v;
+                    }
+                }
+                // one warp per quarter: the direction (under way with the rows) and p.q
+                double pv[ND];
+                const int64_t i0 = (w.node0 + lane) * ND;
+                const bool dir = tid % QT < 32 && have && lane < nn;
+                if (dir) {
+#pragma unroll
+                    for (int d = 0; d < ND; d++) {
+                        if (it == 0) {
+                            pv[d] = pn[i0 + d];
+                        } else {
+                            pv[d] = S.pres_idx[i0 + d] >= 0 ? 0.0 : fma(beta, po[i0 + d], W.z[i0 + d]);
+                            pn[i0 + d] = pv[d];
+                        }
+                        if (keep < WIDE_KEEP) pq_own[2 * keep * 32 * ND + lane * ND + d] = pv[d];
+                    }
+                }
+                __syncthreads();
+                if (tid % QT < 32 && have) {
+                    double v = dir ? node_dot(S.pres_idx + i0, ND, pv, qs + (g * 32 + lane) * ND) : 0.0;
+                    v = warp_tree<false>(v);
+                    if (lane == 0) W.part_pq[w.part] = v;
+                }
+                if (t0 + QPP < len) __syncthreads();
+            }
+            if (rn + 1 < nruns) __syncthreads();
+        }
+        if (it >= W.budget) return;
+        if (!barrier()) return;
+        const unsigned ndone = ctl[1];
+        if (ndone >= (unsigned)nactive || (s == 0 && ndone >= (unsigned)W.stop)) {
+            if (s == 1)  // (every problem has finished)
+                for (int rn = 0; rn < nruns; rn++)
+                    if (runs[rn].off == 0 && tid == 0) {
+                        const int p = runs[rn].prob;
+                        S.pcg_active[p] = 0;
+                        W.rho[p] = runs[rn].rho;
+                        W.iters[p] = runs[rn].iters;
+                    }
+            return;
+        }
+        // ---- B: x, r, z
+        for (int rn = 0; rn < nruns; rn++) {
+            const WideRun& run = runs[rn];
+            if (!run.active) continue;
+            const int len = run.len, first = run.first;
+            if (tid < CHN) total(W.part_pq, run.c0, run.c1, sh, tid);
+            __syncthreads();
+            const double pq = quarters<false>(sh[0], sh[1], sh[2], sh[3]);
+            const double alpha = (pq != 0.0) ? run.rho / pq : 0.0;
+            for (int t = wid; t < len; t += NW) {
+                const WideQuarter& w = quarter(run, t);
+                const int keep = first + t;
+                double rz = 0.0, r2 = 0.0;
+                if (lane < w.nn) {
+                    const int64_t node = w.node0 + lane, i0 = node * ND;
+                    const double* p = keep < WIDE_KEEP ? pq_own + 2 * keep * 32 * ND + lane * ND : pn + i0;
+                    const double* q = keep < WIDE_KEEP ? pq_own + (2 * keep + 1) * 32 * ND + lane * ND : W.q + i0;
+                    node_update(S.pres_idx + i0, ND, alpha, p, q, W.binv + node * ND * ND, W.x + i0, W.r + i0, W.z + i0,
+                                rz, r2);
+                }
+                rz = warp_tree<false>(rz);
+                r2 = warp_tree<false>(r2);
+                if (lane == 0) {
+                    W.part_rz[w.part] = rz;
+                    W.part_rr[w.part] = r2;
+                }
+            }
+            if (rn + 1 < nruns) __syncthreads();  // sh
+        }
+        // before phase C the flags stand still: every WIDE_DEAL iterations the quarters are dealt again,
+        // without the problems that both parities name finished (read before the barrier, since a block
+        // past it may write; p, q are not kept across it)
+        if (it > 0 && it % WIDE_DEAL == 0)
+            deal([&](int p) { return (S.pcg_active[p] | S.pcg_active[S.np + p]) != 0; }, s);
+        if (!barrier()) return;
     }
 }
 
@@ -773,7 +1143,7 @@ __global__ void fill_masked_kernel(SolverArgs S, const uint8_t* flag, double* v,
 
 // ---- device-resident load step (pms_batch_solve_step_graph) --------------------------------
 // One CUDA graph per load step: a conditional WHILE over Newton iterations, each one the element pass,
-// the residual test, the PCG start, a nested WHILE over PCG iterations (batch-wide engine), the
+// the residual test, the PCG start, the PCG (batch-wide engine: one cooperative kernel, or a nested WHILE), the
 // completion and the update.  The per-problem sequencing of pms_batch_tick (and of
 // SolverImplicit::iterate, src/fem/solver_implicit.rs:187-272) runs in these controller kernels
 // instead of on the host; each problem's arithmetic is the same kernels' and gives the same bits.
@@ -805,7 +1175,7 @@ __global__ void step_pre_elem_kernel(int np, const uint8_t* phase, uint8_t* pmod
 }
 
 // after the residual: element errors, NaN/Inf, convergence on max|R|, or on to the linear solve
-__global__ void step_post_resid_kernel(int np, cudaGraphConditionalHandle pcg_loop, double tol_rr,
+__global__ void step_post_resid_kernel(int np, cudaGraphConditionalHandle pcg_loop, int use_loop, double tol_rr,
                                        const unsigned long long* perr, const double* norm, uint8_t* phase,
                                        uint8_t* active, uint8_t* first, const int32_t* it, int32_t* st, int32_t* cnt,
                                        double* lastnorm) {
@@ -838,7 +1208,7 @@ __global__ void step_post_resid_kernel(int np, cudaGraphConditionalHandle pcg_lo
         active[p] = solve;
     }
     __syncthreads();
-    if (threadIdx.x == 0) cudaGraphSetConditional(pcg_loop, any ? 1u : 0u);
+    if (use_loop && threadIdx.x == 0) cudaGraphSetConditional(pcg_loop, any ? 1u : 0u);
 }
 
 __global__ void step_cond_pcg_kernel(cudaGraphConditionalHandle pcg_loop, const int32_t* nactive) {
@@ -907,6 +1277,9 @@ struct pms_batch {
     double *d_part_a = nullptr, *d_part_b = nullptr, *d_part_c = nullptr;
     double *d_rho = nullptr, *d_r0 = nullptr, *d_norm = nullptr, *d_rel = nullptr;
     int32_t *d_iters = nullptr, *d_nactive = nullptr;
+    double *d_p1 = nullptr, *d_part_q = nullptr;  // batch-wide engine: second direction, r.z and r.r quarters
+    unsigned* d_ctl = nullptr;                    // its barrier, finished problems, failure flag
+    WideQuarter* d_quarter = nullptr;             // its units of work
     int64_t* d_queue = nullptr;    // work queue of the element pass: 4 arrays of np + 1
     unsigned long long* d_perr = nullptr;  // per problem: key of its element error in the last pass
     // device-resident load step
@@ -922,11 +1295,11 @@ struct pms_batch {
     cudaEvent_t ev_fork = nullptr, ev_cls[5] = {};
     int cls_off[6] = {};
     int team_cmax = 8;
+    cudaGraphExec_t graph = nullptr;
+    int graph_iters_captured = 0;
     bool fit_teams = true;         // team sizes follow the load (until a tuning is set)
     int budget_factor = 1;         // PCG budget of a tick, in units of the tuned one
     int team_slots[5] = {};        // teams of 1, 2, 4, 8, 16 CTAs that the device holds at once
-    cudaGraphExec_t graph = nullptr;
-    int graph_iters_captured = 0;
     std::string last_error;
     int64_t launches = 0;
     int64_t pcg_total = 0;
@@ -993,12 +1366,12 @@ void launch_spmv(pms_batch* b, const double* x, double* y, const uint8_t* flag, 
 
 // Appends a kernel node (after `dep`, if any) to graph g; args point at the argument values.
 cudaError_t add_kernel_node(cudaGraph_t g, cudaGraphNode_t* node, cudaGraphNode_t dep, void* fn, unsigned grid,
-                            unsigned block, void** args) {
+                            unsigned block, void** args, size_t smem) {
     cudaKernelNodeParams kp = {};
     kp.func = fn;
     kp.gridDim = dim3(grid);
     kp.blockDim = dim3(block);
-    kp.sharedMemBytes = 0;
+    kp.sharedMemBytes = (unsigned)smem;
     kp.kernelParams = args;
     kp.extra = nullptr;
     return cudaGraphAddKernelNode(node, g, dep ? &dep : nullptr, dep ? 1 : 0, &kp);
@@ -1035,9 +1408,9 @@ int ensure_graph(pms_batch* b) {
         void* a3[] = {&b->S, &par, &b->d_part_a, &b->d_part_b, &b->d_rho, &b->d_r0, &rtol, &max_iter,
                       &b->d_iters, &b->d_z, &b->d_p, &b->d_nactive};
         cudaGraphNode_t n1, n2, n3;
-        ok = add_kernel_node(g, &n1, prev, spmv, 4 * nch, qthreads, a1) == cudaSuccess &&
-             add_kernel_node(g, &n2, n1, (void*)pcg_update_kernel, nch, CHN, a2) == cudaSuccess &&
-             add_kernel_node(g, &n3, n2, (void*)pcg_beta_direction_kernel, nch, CHN, a3) == cudaSuccess;
+        ok = add_kernel_node(g, &n1, prev, spmv, 4 * nch, qthreads, a1, 0) == cudaSuccess &&
+             add_kernel_node(g, &n2, n1, (void*)pcg_update_kernel, nch, CHN, a2, 0) == cudaSuccess &&
+             add_kernel_node(g, &n3, n2, (void*)pcg_beta_direction_kernel, nch, CHN, a3, 0) == cudaSuccess;
         prev = n3;
         b->launches += 3;
     }
@@ -1049,6 +1422,72 @@ int ensure_graph(pms_batch* b) {
     cudaGraphDestroy(g);
     b->graph_iters_captured = gi;
     return PMS_OK;
+}
+
+// Launch shape and arguments of the cooperative batch-wide engine.  grid: as many blocks as the device holds, at most
+// one per group of quarters worked on together.
+struct WideShape {
+    const void* kern;
+    unsigned grid;
+    size_t smem;
+    int maxruns, maxshare;  // of a block
+};
+
+WideShape wide_shape(const pms_batch* b) {
+    const bool two = tpr_of(b->v.nd) == 8;
+    WideShape s;
+    s.kern = two ? (const void*)pcg_wide_kernel<8> : (const void*)pcg_wide_kernel<16>;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t groups = std::max<int64_t>(1, two ? 2 * b->nchunk : 4 * b->nchunk);
+    int64_t grid = std::min<int64_t>(groups, sms);  // one block per SM, so that two batches can run side by side
+    // a block's share, and the problems it spans at most (each has four quarters at least)
+    s.maxshare = (int)((4 * b->nchunk + grid - 1) / grid) + 1;
+    s.maxruns = s.maxshare / 4 + 3;
+    s.smem = wide_smem_bytes(b->v.nd, s.maxruns, s.maxshare);
+    s.grid = (unsigned)grid;
+    return s;
+}
+
+WideArgs wide_args(const pms_batch* b, int budget, int stop) {
+    WideArgs w;
+    w.quarter = b->d_quarter;
+    w.bcol = b->v.d_bcol;
+    w.val = b->d_csr;
+    w.binv = b->d_binv;
+    w.p0 = b->d_p;
+    w.p1 = b->d_p1;
+    w.q = b->d_q;
+    w.x = b->d_x;
+    w.r = b->d_r;
+    w.z = b->d_z;
+    w.part_pq = b->d_part_c;
+    w.part_rz = b->d_part_q;
+    w.part_rr = b->d_part_q + 4 * b->nchunk;
+    w.rho = b->d_rho;
+    w.r0 = b->d_r0;
+    w.iters = b->d_iters;
+    w.ctl = b->d_ctl;
+    w.rtol = b->cfg.pcg_rtol;
+    w.max_iter = b->cfg.pcg_max_iterations;
+    w.budget = (budget + 1) & ~1;
+    w.stop = stop;
+    return w;
+}
+
+// Up to `budget` iterations of the active problems on the batch-wide engine; it ends early, at an even
+// iteration, once `stop` problems have finished.
+int launch_wide(pms_batch* b, int budget, int stop, cudaStream_t st) {
+    const WideShape s = wide_shape(b);
+    WideArgs w = wide_args(b, budget, stop);
+    int maxruns = s.maxruns, maxshare = s.maxshare;
+    void* args[] = {&b->S, &w, &maxruns, &maxshare};
+    cudaMemsetAsync(b->d_ctl, 0, 3 * sizeof(unsigned), st);
+    b->launches++;
+    return cudaLaunchCooperativeKernel(s.kern, dim3(s.grid), dim3(WIDE_THREADS), args, s.smem, st) == cudaSuccess
+               ? PMS_OK
+               : bfail(b, PMS_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
 }
 
 constexpr int NCLASS = 5;  // team sizes 1, 2, 4, 8, 16
@@ -1102,7 +1541,11 @@ int team_setup(int* cmax) {
     std::lock_guard<std::mutex> lock(m);
     if (cached < 0) {
         const bool ok = team_attrs_t<256, 8>() && team_attrs_t<256, 16>() && team_attrs_t<512, 8>() &&
-                        team_attrs_t<512, 16>() && team_attrs_t<1024, 8>() && team_attrs_t<1024, 16>();
+                        team_attrs_t<512, 16>() && team_attrs_t<1024, 8>() && team_attrs_t<1024, 16>() &&
+                        cudaFuncSetAttribute(pcg_wide_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)TEAM_SMEM_LIMIT) == cudaSuccess &&
+                        cudaFuncSetAttribute(pcg_wide_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)TEAM_SMEM_LIMIT) == cudaSuccess;
         if (!ok) return PMS_ERR_CUDA;
         int c = 16;
         for (int nd = 2; nd <= 3; nd++) {
@@ -1158,7 +1601,7 @@ void pcg_start(pms_batch* b) {
 }
 
 // PCG iterations of every solving problem: one team launch per team size (each on its own stream)
-// and the batch-wide engine (graph launches on the handle's stream) run side by side.  The team
+// and the batch-wide engine (cooperative launches on the handle's stream) run side by side.  The team
 // lists are in b->h_list, grouped by team size (b->cls_off).  The batch-wide loop keeps going while
 // a team launch is busy; once they are idle, it stops when an eighth of its problems (at least
 // one) have finished or after `budget` iterations.  `exact` runs exactly `budget` iterations on
@@ -1187,19 +1630,34 @@ int pcg_phase(pms_batch* b, int nteam, int nwide, int budget, bool exact) {
         return false;
     };
     if (nwide > 0) {
-        int rc = ensure_graph(b);
-        if (rc) return rc;
+        // cooperative: eight times the graph_iters of the tuning per launch and wait of the host
+        const bool coop = b->nchunk <= WIDE_MAX_CHUNKS;
+        if (!coop) {
+            int rc = ensure_graph(b);
+            if (rc) return rc;
+        }
+        const int per = !coop ? b->graph_iters_captured
+                              : (exact ? budget : 8 * std::max(2, b->tune.graph_iters + (b->tune.graph_iters & 1)));
         int32_t nact = nwide;
-        const int32_t stop_at = nwide - std::max(1, nwide / 8);
+        const int stop_at = nwide - std::max(1, nwide / 8);
         for (int64_t done = 0; nact > 0;) {
             if (exact && done >= budget) break;
-            if (cudaGraphLaunch(b->graph, st) != cudaSuccess) return bfail(b, PMS_ERR_CUDA, "graph launch failed");
-            done += b->graph_iters_captured;
+            if (!coop) {
+                if (cudaGraphLaunch(b->graph, st) != cudaSuccess) return bfail(b, PMS_ERR_CUDA, "graph launch failed");
+            } else {
+                int rc = launch_wide(b, per, nteam > 0 || exact ? INT32_MAX : std::max(1, nact - stop_at), st);
+                if (rc) return rc;
+            }
+            done += per;
             if (exact) continue;
-            cudaMemcpyAsync(&nact, b->d_nactive, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+            unsigned ctl[3] = {0, 0, 0};
+            if (coop) cudaMemcpyAsync(ctl, b->d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost, st);
+            else cudaMemcpyAsync(&nact, b->d_nactive, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
             b->host_syncs++;
             if (cudaStreamSynchronize(st) != cudaSuccess)
                 return bfail(b, PMS_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
+            if (ctl[2]) return bfail(b, PMS_ERR_ORDER, "PCG: a wait for the other blocks timed out (internal error)");
+            nact -= (int)ctl[1];
             if (!teams_busy() && (nact <= stop_at || done >= budget)) break;
         }
     }
@@ -1418,7 +1876,9 @@ int pms_batch_create(pms_elements* el, int32_t nproblem, const int64_t* point_pt
               b->alloc(&b->d_rho, 2 * (size_t)nproblem) && b->alloc(&b->d_r0, nproblem) &&
               b->alloc(&b->d_norm, nproblem) && b->alloc(&b->d_rel, nproblem) &&
               b->alloc(&b->d_iters, 2 * (size_t)nproblem) &&
-              b->alloc(&b->d_nactive, 1) && b->alloc(&b->d_queue, 4 * ((size_t)nproblem + 1)) &&
+              b->alloc(&b->d_nactive, 1) && b->alloc(&b->d_p1, n) && b->alloc(&b->d_part_q, 8 * (size_t)b->nchunk) && b->alloc(&b->d_ctl, 4) &&
+              b->alloc(&b->d_quarter, 4 * (size_t)b->nchunk) &&
+              b->alloc(&b->d_queue, 4 * ((size_t)nproblem + 1)) &&
               b->alloc(&b->d_perr, (size_t)nproblem) && b->alloc(&b->d_phase, nproblem) &&
               b->alloc(&b->d_sel, nproblem) && b->alloc(&b->d_zero_engine, nproblem) &&
               b->alloc(&b->d_st, nproblem) && b->alloc(&b->d_cnt, nproblem) && b->alloc(&b->d_pcgsum, nproblem) &&
@@ -1468,6 +1928,8 @@ int pms_batch_create(pms_elements* el, int32_t nproblem, const int64_t* point_pt
     b->pnch.assign(nproblem, 0);
     for (int p = 0; p < nproblem; p++) b->pnch[p] = pchunk[p + 1] - pchunk[p];
     count_team_slots(b);
+    wide_quarters_kernel<<<grid_of(32 * 4 * b->nchunk), 256>>>(4 * b->nchunk, b->d_chunk_node0, b->d_chunk_nnode,
+                                                                b->v.d_bptr, b->d_quarter);
     if (assign_engines(b) || cudaDeviceSynchronize() != cudaSuccess) {
         delete b;
         return PMS_ERR_CUDA;
@@ -1708,14 +2170,30 @@ struct GraphChain {
     cudaGraphNode_t prev = nullptr;
     bool ok = true;
     int nodes = 0;
-    void kernel(const void* fn, unsigned grid, unsigned block, void** args) {
+    void kernel(const void* fn, unsigned grid, unsigned block, void** args, size_t smem = 0, bool cooperative = false) {
         if (!ok) return;
         cudaGraphNode_t n;
-        ok = add_kernel_node(g, &n, prev, (void*)fn, grid, block, args) == cudaSuccess;
+        ok = add_kernel_node(g, &n, prev, (void*)fn, grid, block, args, smem) == cudaSuccess;
+        if (ok && cooperative) {
+            cudaLaunchAttributeValue v = {};
+            v.cooperative = 1;
+            ok = cudaGraphKernelNodeSetAttribute(n, cudaLaunchAttributeCooperative, &v) == cudaSuccess;
+        }
         if (ok) {
             prev = n;
             nodes++;
         }
+    }
+    void zero(unsigned* p, size_t words) {
+        if (!ok) return;
+        cudaMemsetParams mp = {};
+        mp.dst = (void*)p;
+        mp.elementSize = 4;
+        mp.width = words;
+        mp.height = 1;
+        cudaGraphNode_t n;
+        ok = cudaGraphAddMemsetNode(&n, g, prev ? &prev : nullptr, prev ? 1 : 0, &mp) == cudaSuccess;
+        if (ok) prev = n;
     }
     // a conditional WHILE node on handle h (created on this graph); returns its body graph
     cudaGraph_t while_node(cudaGraphConditionalHandle h) {
@@ -1745,6 +2223,8 @@ int build_step_graph(pms_batch* b) {
     S.engine = b->d_zero_engine;  // every PCG on the batch-wide engine (the engines give the same bits)
     double tol_rr = b->cfg.tol_rr_abs, tol_mdu = b->cfg.tol_mdu_rel, rtol = b->cfg.pcg_rtol;
     int32_t max_it = b->cfg.n_max_iterations, max_pcg = b->cfg.pcg_max_iterations;
+    const bool coop = b->nchunk <= WIDE_MAX_CHUNKS;
+    int use_loop = coop ? 0 : 1;
     int zero = 0;
     bool no_mask = false;
     const unsigned nch = (unsigned)b->nchunk;
@@ -1765,7 +2245,7 @@ int build_step_graph(pms_batch* b) {
     cudaGraph_t B1 = top.while_node(hN);
     GraphChain body{B1};
     body.ok = top.ok;
-    if (body.ok) body.ok = cudaGraphConditionalHandleCreate(&hP, B1, 0, 0) == cudaSuccess;
+    if (body.ok && !coop) body.ok = cudaGraphConditionalHandleCreate(&hP, B1, 0, 0) == cudaSuccess;
     // element pass of the problems that start a step or continue it
     int ct = b->cfg.constant_tangent ? 1 : 0;
     void* a_pre[] = {&np, &b->d_phase, &b->d_pmode, &b->d_upd, &b->d_active, &b->d_it, &b->d_perr, &ct};
@@ -1780,7 +2260,7 @@ int build_step_graph(pms_batch* b) {
     body.kernel((const void*)residual_kernel, nch, CHN, a_res);
     void* a_fin_n[] = {&np, &b->d_pchunk, &b->d_part_a, &b->d_norm, &zero};
     body.kernel((const void*)finalize_kernel, grid_of(np, 128), 128, a_fin_n);
-    void* a_post[] = {&np, &hP, &tol_rr, &b->d_perr, &b->d_norm, &b->d_phase, &b->d_active, &b->d_first, &b->d_it,
+    void* a_post[] = {&np, &hP, &use_loop, &tol_rr, &b->d_perr, &b->d_norm, &b->d_phase, &b->d_active, &b->d_first, &b->d_it,
                       &b->d_st, &b->d_cnt, &b->d_lastnorm};
     body.kernel((const void*)step_post_resid_kernel, 1, 1024, a_post);
     // PCG start (block Jacobi, prescribed increments, r = R_f - K_fp mdu_p, scalars)
@@ -1795,25 +2275,37 @@ int build_step_graph(pms_batch* b) {
     void* a_is[] = {&np, &b->d_active, &b->d_zero_engine, &b->d_pchunk, &b->d_part_a, &b->d_part_b, &b->d_rho,
                     &b->d_r0, &b->d_pcg_active, &b->d_cta_active, &b->d_iters};
     body.kernel((const void*)pcg_init_scalars_kernel, (unsigned)np, CHN, a_is);
-    // PCG iterations, two per pass (the scalars are double-buffered by iteration parity)
-    cudaGraph_t B2 = body.while_node(hP);
-    GraphChain pcg{B2};
-    pcg.ok = body.ok;
-    int par0 = 0, par1 = 1;
-    for (int k = 0; k < 2; k++) {
-        int* par = k ? &par1 : &par0;
-        void* a1[] = {&S, par, (void*)&bptr, (void*)&bcol, (void*)&csr, &b->d_p, &b->d_q, &b->d_part_c};
-        pcg.kernel(spmv_dot, 4 * nch, qthreads, a1);
-        void* a2[] = {&S, par, &b->d_part_c, &b->d_rho, &b->d_p, &b->d_q, &b->d_binv, &b->d_x, &b->d_r, &b->d_z,
-                      &b->d_part_a, &b->d_part_b, &b->d_nactive};
-        pcg.kernel((const void*)pcg_update_kernel, nch, CHN, a2);
-        void* a3[] = {&S, par, &b->d_part_a, &b->d_part_b, &b->d_rho, &b->d_r0, &rtol, &max_pcg, &b->d_iters, &b->d_z,
-                      &b->d_p, &b->d_nactive};
-        pcg.kernel((const void*)pcg_beta_direction_kernel, nch, CHN, a3);
+    int nodes = 0;
+    if (coop) {
+        // the PCG of every problem to its end
+        const WideShape wshape = wide_shape(b);
+        WideArgs wargs = wide_args(b, b->cfg.pcg_max_iterations + 2, INT32_MAX);
+        int wruns = wshape.maxruns, wshare = wshape.maxshare;
+        void* a_pcg[] = {&S, &wargs, &wruns, &wshare};
+        body.zero(b->d_ctl, 2);  // the failure flag stays for the host
+        body.kernel(wshape.kern, wshape.grid, WIDE_THREADS, a_pcg, wshape.smem, true);
+    } else {
+        // PCG iterations, two per pass (the scalars are double-buffered by iteration parity)
+        cudaGraph_t B2 = body.while_node(hP);
+        GraphChain pcg{B2};
+        pcg.ok = body.ok;
+        int par0 = 0, par1 = 1;
+        for (int k = 0; k < 2; k++) {
+            int* par = k ? &par1 : &par0;
+            void* a1[] = {&S, par, (void*)&bptr, (void*)&bcol, (void*)&csr, &b->d_p, &b->d_q, &b->d_part_c};
+            pcg.kernel(spmv_dot, 4 * nch, qthreads, a1);
+            void* a2[] = {&S, par, &b->d_part_c, &b->d_rho, &b->d_p, &b->d_q, &b->d_binv, &b->d_x, &b->d_r, &b->d_z,
+                          &b->d_part_a, &b->d_part_b, &b->d_nactive};
+            pcg.kernel((const void*)pcg_update_kernel, nch, CHN, a2);
+            void* a3[] = {&S, par, &b->d_part_a, &b->d_part_b, &b->d_rho, &b->d_r0, &rtol, &max_pcg, &b->d_iters, &b->d_z,
+                          &b->d_p, &b->d_nactive};
+            pcg.kernel((const void*)pcg_beta_direction_kernel, nch, CHN, a3);
+        }
+        void* a_cp[] = {&hP, &b->d_nactive};
+        pcg.kernel((const void*)step_cond_pcg_kernel, 1, 1, a_cp);
+        body.ok = body.ok && pcg.ok;
+        nodes += pcg.nodes;
     }
-    void* a_cp[] = {&hP, &b->d_nactive};
-    pcg.kernel((const void*)step_cond_pcg_kernel, 1, 1, a_cp);
-    body.ok = body.ok && pcg.ok;
     // completion: mdu, multiplier increments, rel(mdu), and the update
     void* a_am[] = {&S, &b->d_x, &b->d_mdu};
     body.kernel((const void*)assemble_mdu_kernel, grid_of(b->ndof), 256, a_am);
@@ -1846,7 +2338,7 @@ int build_step_graph(pms_batch* b) {
         return bfail(b, PMS_ERR_CUDA, "load-step graph construction failed");
     }
     cudaGraphDestroy(G);
-    b->launches += top.nodes + body.nodes + pcg.nodes + 1;
+    b->launches += top.nodes + body.nodes + nodes + 1;
     return PMS_OK;
 }
 }  // namespace
@@ -1865,7 +2357,10 @@ int pms_batch_solve_step_graph(pms_batch* b, const double* c_values, const uint8
     cudaStream_t st = b->v.stream;
     if (b->npres > 0) cudaMemcpyAsync(b->d_c, c_values, b->npres * 8, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b->d_sel, active, np, cudaMemcpyHostToDevice, st);
+    cudaMemsetAsync(b->d_ctl, 0, 3 * sizeof(unsigned), st);
     if (cudaGraphLaunch(b->step_graph, st) != cudaSuccess) return bfail(b, PMS_ERR_CUDA, "load-step graph launch failed");
+    unsigned ctl[3] = {0, 0, 0};
+    cudaMemcpyAsync(ctl, b->d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost, st);
     std::vector<int32_t> cnt(np), stv(np), pcg(np), itv(np);
     std::vector<double> norm(np);
     cudaMemcpyAsync(cnt.data(), b->d_cnt, np * 4, cudaMemcpyDeviceToHost, st);
@@ -1874,6 +2369,7 @@ int pms_batch_solve_step_graph(pms_batch* b, const double* c_values, const uint8
     cudaMemcpyAsync(itv.data(), b->d_it, np * 4, cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(norm.data(), b->d_lastnorm, np * 8, cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return bfail(b, PMS_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
+    if (ctl[2]) return bfail(b, PMS_ERR_ORDER, "PCG: a wait for the other blocks timed out (internal error)");
     rc = elements_status(b->el);  // element errors are per problem (in stv); anything else is fatal
     if (rc != PMS_OK && rc != PMS_ERR_ZERO_SIGMA_D && rc != PMS_ERR_ZERO_NORM_S && rc != PMS_ERR_JACOBIAN) return rc;
     for (int p = 0; p < np; p++) {

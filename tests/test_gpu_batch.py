@@ -270,3 +270,24 @@ def test_team_sizes_that_follow_the_load_give_the_same_bits():
         for x, y in zip(ra, rb):
             assert np.array_equal(x, y)
         assert np.array_equal(a.u(), b.u())
+
+
+@pytest.mark.parametrize("nx,count", [(3, 1), (12, 2), (26, 9), (40, 9)])
+def test_batch_wide_engines_give_the_same_bits(nx, count):
+    """The batch-wide engine is one cooperative kernel up to 104 chunks (one problem of a quarter chunk,
+    blocks that hold runs of several problems, problems that finish and leave the deal) and a CUDA graph
+    of three kernels beyond (the last case): the iterates of the teams, host-sequenced and with the
+    Newton loop on the device."""
+    from pmsim_b200.batch import BatchSolver
+    probs = [footing(nx + i % 3, max(2, (nx + i) // 2), 1e4 * (1 + 0.2 * i), 9.0 + i, 1.0, nsteps=2) for i in range(count)]
+    out = []
+    for mode in ("teams", "wide", "device"):
+        b = BatchSolver(probs)
+        if mode == "wide":
+            b.set_tuning(**{**b.tuning(), "team_max_ndof": 0})
+        b.solve(device_loop=mode == "device", on_fail="drop")
+        out.append((b.u(), *b.elements.get_state(), b.history, b.pcg_history))
+    for o in out[1:]:
+        for x, y in zip(out[0][:4], o[:4]):
+            assert np.array_equal(x, y)
+        assert out[0][4:] == o[4:]
