@@ -237,6 +237,10 @@ element_kernel(ElemArgs A) {
             Ns[m * 32 + p] = A.tab[ng * NE + ng + i];
         }
     __syncthreads();
+    if constexpr (!CSR) {
+        let_next_start();
+        wait_for_previous();
+    }
 
     // the warps of one cell meet at a named barrier (id 1 + cell slot)
     auto cell_sync = [&]() {
@@ -1015,6 +1019,10 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
             Ns[m * 16 + p] = A.tab[ng * NE + ng + i];
         }
     __syncthreads();
+    if constexpr (!CSR) {
+        let_next_start();
+        wait_for_previous();
+    }
 
     // this lane's tile (ti <= tj), row-major over the upper triangle of node groups
     int ti = -1, tj = -1;
@@ -1605,6 +1613,8 @@ template <int ND>
 __global__ void __launch_bounds__(256) f_gather_kernel(int64_t npoint, const int64_t* __restrict__ inc_ptr,
                                                        const int32_t* __restrict__ inc,
                                                        const double* __restrict__ fe, double* __restrict__ ff) {
+    let_next_start();
+    wait_for_previous();
     for (int64_t A = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; A < npoint;
          A += (int64_t)gridDim.x * blockDim.x) {
         double s[ND];
@@ -1856,7 +1866,12 @@ void launch_elem2d_lpc(pms_elements* h, const ElemArgs& a, cudaStream_t st) {
     if (h) blocks = std::min<int64_t>(blocks, launch_plan(h, (const void*)kern, smem, WPB2 * 32));
     else allow_dynamic_smem((const void*)kern);
     if (CSR) cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), st);
-    kern<<<(unsigned)std::max<int64_t>(blocks, 1), WPB2 * 32, smem, st>>>(a);
+    if (CSR) {
+        kern<<<(unsigned)std::max<int64_t>(blocks, 1), WPB2 * 32, smem, st>>>(a);
+    } else {
+        void* args[] = {(void*)&a};
+        launch_overlapped(a.overlap, (const void*)kern, std::max<int64_t>(blocks, 1), WPB2 * 32, smem, st, args);
+    }
 }
 
 template <int NN, int UPD, bool DOF, bool DOK, bool CSR>
@@ -1882,7 +1897,12 @@ void launch_elem_t(pms_elements* h, const ElemArgs& a) {
     int64_t blocks = (a.ncell + cells_per_block(NN) - 1) / cells_per_block(NN);
     blocks = std::min<int64_t>(blocks, launch_plan(h, (const void*)kern, h->smem_bytes, WPB * 32));
     if (CSR) cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), h->stream);
-    kern<<<(unsigned)blocks, WPB * 32, h->smem_bytes, h->stream>>>(a);
+    if (CSR) {
+        kern<<<(unsigned)blocks, WPB * 32, h->smem_bytes, h->stream>>>(a);
+    } else {
+        void* args[] = {(void*)&a};
+        launch_overlapped(a.overlap, (const void*)kern, blocks, WPB * 32, h->smem_bytes, h->stream, args);
+    }
 }
 
 // upd: UPD_NONE / UPD_CURRENT / UPD_BACKUP; csr: direct assembly into a.csr / a.ff (else dense
@@ -1998,6 +2018,17 @@ static int64_t value_offset(const pms_elements* h, int64_t A) {
     return h->sym == PMS_SYM_FULL ? (int64_t)h->nd * h->nd * h->pat.bptr[A] : h->tbase[A];
 }
 
+int64_t gather_blocks(const GatherShape& g, int64_t nrow) {
+    const int64_t rows = (int64_t)g.rows * g.wpb;
+    return (nrow + rows - 1) / rows;
+}
+
+// Whether the gather of every row is one wave, so that the call's kernels overlap their launches.
+bool gather_is_one_wave(pms_elements* h) {
+    const GatherShape g = gather_shape(h->kind, h->sym != PMS_SYM_FULL, h->pat.nbmax);
+    return gather_blocks(g, h->npoint) <= launch_plan(h, g.kern, g.smem, 32 * g.wpb, false);
+}
+
 // CSR gather of the block rows [node0, node0 + nrow) into the handle's storage of the values, and
 // their rows of R (ff, nullable)
 void launch_kk_gather(pms_elements* h, double* csr, double* ff, int64_t node0, int64_t nrow) {
@@ -2017,20 +2048,18 @@ void launch_kk_gather(pms_elements* h, double* csr, double* ff, int64_t node0, i
     P.kdiag = h->d_kdiag;
     P.tbase = h->d_tbase;
     const GatherShape g = gather_shape(h->kind, h->sym != PMS_SYM_FULL, h->pat.nbmax);
-    const int64_t rows = (int64_t)g.rows * g.wpb;
-    const int64_t blocks = std::min<int64_t>((nrow + rows - 1) / rows, launch_plan(h, g.kern, g.smem, 32 * g.wpb, false));
+    const int64_t want = gather_blocks(g, nrow), resident = launch_plan(h, g.kern, g.smem, 32 * g.wpb, false);
+    const int64_t blocks = std::min(want, resident);
     void* args[] = {&P};
-    cudaLaunchKernel(g.kern, dim3((unsigned)std::max<int64_t>(blocks, 1)), dim3((unsigned)(32 * g.wpb)), args,
-                     (size_t)g.smem, h->stream);
+    launch_overlapped(want <= resident, g.kern, std::max<int64_t>(blocks, 1), 32 * g.wpb, g.smem, h->stream, args);
     h->launches++;
 }
 
 void launch_f_gather(pms_elements* h, double* ff) {
-    const int64_t n = h->npoint;
-    if (h->nd == 2)
-        f_gather_kernel<2><<<grid_1d(n), 256, 0, h->stream>>>(n, h->d_inc_ptr, h->d_inc, h->d_fe, ff);
-    else
-        f_gather_kernel<3><<<grid_1d(n), 256, 0, h->stream>>>(n, h->d_inc_ptr, h->d_inc, h->d_fe, ff);
+    int64_t n = h->npoint;
+    void* args[] = {&n, &h->d_inc_ptr, &h->d_inc, &h->d_fe, &ff};
+    launch_overlapped(gather_is_one_wave(h), h->nd == 2 ? (const void*)f_gather_kernel<2> : (const void*)f_gather_kernel<3>, grid_1d(n), 256, 0,
+                      h->stream, args);
     h->launches++;
 }
 
@@ -2430,6 +2459,7 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
         if (rc) return rc;
     }
     ElemArgs a = make_args(h, d_ddu);
+    a.overlap = !direct && (dof || dok) && gather_is_one_wave(h);
     if (direct) {
         a.csr = d_csr;
         a.ff = d_ff;
