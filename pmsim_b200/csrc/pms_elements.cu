@@ -933,10 +933,13 @@ element_kernel(ElemArgs A) {
 // in element_kernel), lane m < nnode owns node m (F_int), and in phase 2 lane t owns tile t of the
 // upper node-pair triangle (2x2 node pairs for Tri6/Qua8/Qua9, single pairs for Tri3/Qua4).  Qua8
 // with 9 points runs three cells of 10 lanes per warp (30 of 32 lanes hold a tile in phase 2).
-// Phase 1 also forms, per integration point and node, h = S g (+ q s_zz e_x) and q = N/r, so
-// phase 2 reads its operands from shared memory with no per-point staging or barrier.  Every
-// entry of K_e and f_e takes the same operations in the same order as in element_kernel, so the
-// kernels give the same bits.  A slot without a cell (ragged end, inactive problem) repeats the
+// Phase 1 also forms q = N/r (axisymmetric) per integration point and node, and h = S g (+ q s_zz e_x)
+// at the plastic points, so phase 2 reads its operands from shared memory with no per-point staging
+// or barrier.  Every entry of K_e takes the same operations in the same order as in element_kernel.
+// The kernel is bound by shared-memory wavefronts (82% of the peak at 245,350 plane-strain Qua8 cells),
+// so operands are read as pairs, strains come from the displacement gradient, and h is neither formed
+// nor stored where nothing reads it: 354 -> 340 us there, and 41.0 -> 39.7 us for the step of 12,960
+// axisymmetric Qua8 cells.  A slot without a cell (ragged end, inactive problem) repeats the
 // group's first cell and writes nothing: all slots run the same loop trips, so the warp-wide syncs
 // below are always reached by all 32 lanes.
 constexpr int WPB2 = 4;      // warps per block
@@ -1130,13 +1133,18 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
                 }
             }
             const int p = hl;
+            const double2* X2 = reinterpret_cast<const double2*>(Xs);
+            const double2* U2 = reinterpret_cast<const double2*>(Us);
             double J[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-            for (int m = 0; m < NN; m++)
-#pragma unroll
-                for (int i = 0; i < 2; i++)
-#pragma unroll
-                    for (int j = 0; j < 2; j++) J[i * 2 + j] = fma(Xs[m * 2 + i], dNs[(m * 2 + j) * 16 + p], J[i * 2 + j]);
+            for (int m = 0; m < NN; m++) {
+                const double2 x = X2[m];
+                const double d0 = dNs[(m * 2) * 16 + p], d1 = dNs[(m * 2 + 1) * 16 + p];
+                J[0] = fma(x.x, d0, J[0]);
+                J[1] = fma(x.x, d1, J[1]);
+                J[2] = fma(x.y, d0, J[2]);
+                J[3] = fma(x.y, d1, J[3]);
+            }
             double Ji[4];
             const double det = inv_jacobian<2>(J, Ji);
             if (!(det > 0.0)) err = E_JACOBIAN;
@@ -1148,6 +1156,7 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
             }
             const double coef = det * ws[p] * (A.axisym ? rad : A.thickness);
             double eps[4] = {0.0, 0.0, 0.0, 0.0};
+            double D[4] = {0.0, 0.0, 0.0, 0.0};  // displacement gradient: sum of u_i g_j
             double* Gp = G + p * GS;
 #pragma unroll
             for (int m = 0; m < NN; m++) {
@@ -1160,13 +1169,18 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
                     g[i] = v;
                 }
                 reinterpret_cast<double2*>(Gp)[m] = make_double2(g[0], g[1]);
+                if (A.axisym) Q[p * NN + m] = Ns[m * 16 + p] / rad;  // N/r
                 if (do_update) {
-                    const double* u = Us + m * 2;
-                    eps[0] += u[0] * g[0];
-                    eps[1] += u[1] * g[1];
-                    eps[3] += SQRT2 * ((u[0] * g[1] + u[1] * g[0]) / 2.0);
+                    const double2 u = U2[m];
+                    D[0] = fma(u.x, g[0], D[0]);
+                    D[1] = fma(u.x, g[1], D[1]);
+                    D[2] = fma(u.y, g[0], D[2]);
+                    D[3] = fma(u.y, g[1], D[3]);
                 }
             }
+            eps[0] = D[0];
+            eps[1] = D[3];
+            eps[3] = (D[1] + D[2]) * INV_SQRT2;  // Mandel: sqrt(2) (D_01 + D_10)/2
             if (A.axisym && do_update)  // out-of-plane strain u_r / r (calculate_strain.rs:36-48)
 #pragma unroll
                 for (int m = 0; m < NN; m++) eps[2] += Us[m * 2] * Ns[m * 16 + p] / rad;
@@ -1174,13 +1188,10 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
                 const int st = ip_update<4>(mc, mc.hh, sig, z, lam, el, eps);
                 if (st != OK && err == OK) err = st;
             }
-            if (DOF) {  // coef * sigma: xx, yy, xy, hoop (axisymmetric), and the radius
-                double* c6 = CS + p * 6;
-                c6[0] = coef * sig[0];
-                c6[1] = coef * sig[1];
-                c6[2] = coef * sig[3] * INV_SQRT2;
-                c6[3] = coef * sig[2];
-                c6[4] = rad;
+            if (DOF) {  // coef * sigma: xx, yy, xy, hoop (axisymmetric)
+                double2* c6 = reinterpret_cast<double2*>(CS + p * 6);
+                c6[0] = make_double2(coef * sig[0], coef * sig[1]);
+                c6[1] = make_double2(coef * sig[3] * INV_SQRT2, coef * sig[2]);
             }
             if (dok_c) {
                 double a, b, s[4];
@@ -1192,26 +1203,20 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
                 t[2] = coef * b;
                 const bool plastic = t[2] != 0.0;
                 const double s00 = s[0], s11 = s[1], s01 = s[3] * INV_SQRT2, szz = s[2];
-                double* Hp = H + p * GS;
-                double* Qp = Q + p * NN;
+                if (plastic) {  // h = S g (+ q s_zz e_x)
+                    double2* Hp = reinterpret_cast<double2*>(H + p * GS);
 #pragma unroll
-                for (int m = 0; m < NN; m++) {
-                    const double2 gm = reinterpret_cast<const double2*>(Gp)[m];
-                    const double g0 = gm.x, g1 = gm.y;
-                    double q = 0.0;  // N/r of node m (axisymmetric)
-                    if (A.axisym) {
-                        q = Ns[m * 16 + p] / rad;
-                        Qp[m] = q;
+                    for (int m = 0; m < NN; m++) {
+                        const double2 gm = reinterpret_cast<const double2*>(Gp)[m];
+                        double h0 = fma(s01, gm.y, s00 * gm.x);
+                        const double h1 = fma(s11, gm.y, s01 * gm.x);
+                        if (A.axisym) h0 = fma(Q[p * NN + m], szz, h0);
+                        Hp[m] = make_double2(h0, h1);
                     }
-                    double h0 = 0.0, h1 = 0.0;  // h = S g (+ q s_zz e_x)
-                    if (plastic) {
-                        h0 = fma(s00, g0, h0);
-                        h0 = fma(s01, g1, h0);
-                        h1 = fma(s01, g0, h1);
-                        h1 = fma(s11, g1, h1);
-                        if (A.axisym) h0 = fma(q, szz, h0);
-                    }
-                    reinterpret_cast<double2*>(Hp)[m] = make_double2(h0, h1);
+                } else if (A.axisym) {  // (the one-pass form reads h at every point)
+                    double2* Hp = reinterpret_cast<double2*>(H + p * GS);
+#pragma unroll
+                    for (int m = 0; m < NN; m++) Hp[m] = make_double2(0.0, 0.0);
                 }
             }
         }
@@ -1243,11 +1248,12 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
         if (DOF && hl < NN) {
             double f[2] = {0.0, 0.0};
             for (int p = 0; p < ng; p++) {
-                const double* c6 = CS + p * 6;
-                const double* g = G + p * GS + hl * 2;
-                f[0] += c6[0] * g[0] + c6[2] * g[1];
-                f[1] += c6[2] * g[0] + c6[1] * g[1];
-                if (A.axisym) f[0] += c6[3] * Ns[hl * 16 + p] / c6[4];
+                const double2 d = reinterpret_cast<const double2*>(CS + p * 6)[0];  // xx, yy
+                const double2 o = reinterpret_cast<const double2*>(CS + p * 6)[1];  // xy, hoop
+                const double2 g = reinterpret_cast<const double2*>(G + p * GS)[hl];
+                f[0] += d.x * g.x + o.x * g.y;
+                f[1] += o.x * g.x + d.y * g.y;
+                if (A.axisym) f[0] += o.y * Q[p * NN + hl];
             }
             if (CSR) {  // kept in the cell's dU slot (free after phase 1) until the scatter
                 Us[hl * 2] = f[0];
