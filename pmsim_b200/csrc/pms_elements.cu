@@ -1,5 +1,6 @@
-// pms_elements.cu -- fused per-element kernels (strain -> return map -> B^T sigma -> B^T D B)
-// and the deterministic CSR / residual gathers, behind the pms_elements_* C ABI.
+// pms_elements.cu -- fused per-element kernels (strain -> return map -> B^T sigma -> B^T D B),
+// the direct assembly and the handle behind the pms_elements_* C ABI (the row gathers: pms_gather.cu;
+// Hex8 and Tet4 with several cells per warp: pms_elements3.cu).
 //
 // Reference calls replaced (pmsim 0.3.0):
 //   ElementSolid::update_secondary_values  src/fem/element_solid.rs:190-224 (+ calculate_strain,
@@ -26,14 +27,13 @@
 // FLOPs per IP and pair (3D): 3 (dot) + 9*3 (entries) + 3 (diagonal) = 33 FMA; per node: J^-T
 // dN (9), h = S g (9), three scaled copies (9).
 //
-// 2D cells (at most 9 nodes) run in element2d_kernel instead: the same arithmetic with several
-// cells per warp (three 10-lane Qua8 cells), so that most lanes hold work.
+// 2D cells (at most 9 nodes) run in element2d_kernel instead, Hex8 and Tet4 in element3_kernel: the
+// same arithmetic with several cells per warp (three 10-lane Qua8 cells), so that most lanes hold work.
 //
-// Assembly: each cell's dense element matrix goes to a scratch buffer ke[cell][NE][NE] (the
-// reference's GenericElement::kke, src/fem/elements.rs:13-14); in kk_gather_kernel a group of
-// nnode lanes owns one block row A of K (32/nnode rows per warp), adds the node-row slabs (a, all
-// b) of the cells incident to A in ascending cell order in shared memory and writes the CSR row
-// once, coalesced.  No atomics: bit-identical on every run.
+// Assembly: each cell's upper node-pair blocks go to a scratch buffer (full matrices, the
+// reference's GenericElement::kke, src/fem/elements.rs:13-14, for the per-cell calls); a gather
+// kernel then sums each block row of K and R over the cells incident to it in ascending cell order
+// and writes it once, coalesced.  No atomics: bit-identical on every run.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -2031,7 +2031,7 @@ int64_t gather_blocks(const GatherShape& g, int64_t nrow) {
 
 // Whether the gather of every row is one wave, so that the call's kernels overlap their launches.
 bool gather_is_one_wave(pms_elements* h) {
-    const GatherShape g = gather_shape(h->kind, h->sym != PMS_SYM_FULL, h->pat.nbmax);
+    const GatherShape g = gather_shape(h->kind, h->sym != PMS_SYM_FULL, false, h->pat.nbmax);
     return gather_blocks(g, h->npoint) <= launch_plan(h, g.kern, g.smem, 32 * g.wpb, false);
 }
 
@@ -2053,8 +2053,14 @@ void launch_kk_gather(pms_elements* h, double* csr, double* ff, int64_t node0, i
     P.sym = h->sym;
     P.kdiag = h->d_kdiag;
     P.tbase = h->d_tbase;
-    const GatherShape g = gather_shape(h->kind, h->sym != PMS_SYM_FULL, h->pat.nbmax);
-    const int64_t want = gather_blocks(g, nrow), resident = launch_plan(h, g.kern, g.smem, 32 * g.wpb, false);
+    // the kernel that loads further ahead, where it still has every row in flight at once
+    GatherShape g = gather_shape(h->kind, h->sym != PMS_SYM_FULL, true, h->pat.nbmax);
+    int64_t want = gather_blocks(g, nrow), resident = launch_plan(h, g.kern, g.smem, 32 * g.wpb, false);
+    if (want > resident) {
+        g = gather_shape(h->kind, h->sym != PMS_SYM_FULL, false, h->pat.nbmax);
+        want = gather_blocks(g, nrow);
+        resident = launch_plan(h, g.kern, g.smem, 32 * g.wpb, false);
+    }
     const int64_t blocks = std::min(want, resident);
     void* args[] = {&P};
     launch_overlapped(want <= resident, g.kern, std::max<int64_t>(blocks, 1), 32 * g.wpb, g.smem, h->stream, args);
@@ -2195,7 +2201,7 @@ int pms_elements_create(const pms_mesh* mesh, const pms_material* materials, int
     }
     h->stream = h->own_stream;
     h->smem_bytes = smem_bytes_for(h->nn, h->nd, h->ng, WPB);
-    // kk_gather: one warp's row buffers (up to 32/nnode rows, each with room for the largest) fit a block
+    // K gather: one warp's row buffers (up to 32/nnode rows, each with room for the largest) fit a block
     if ((int64_t)(32 / h->nn) * std::max(h->pat.nbmax, 1) * h->nd * h->nd * 8 > 200 * 1024) {
         delete h;
         return PMS_ERR_TOO_LARGE;

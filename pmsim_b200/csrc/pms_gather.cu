@@ -47,15 +47,22 @@ template <int NN> struct Gather3 {
     static constexpr int ROWS = NN >= 13 ? 1 : 3;
     static constexpr int BPI = 3 / ROWS;              // blocks at a time
     static constexpr int NIT = (NN + BPI - 1) / BPI;  // blocks per lane and incidence
-    static constexpr int NB = ROWS == 1 ? 2 : 1;      // incidences loaded before they are added
+    static constexpr bool FEW = NN != 10;             // has a kernel for few rows (no mesh of Tet10 to measure)
     static constexpr int CL = ROWS == 1 ? 27 : 9;     // lanes that hold a row's incidences
 };
 
-template <int NN, bool TRI>
-__global__ void __launch_bounds__(GATHER_WARPS * 32, 3) gather3_kernel(GatherArgs P) {
+// NB incidences are loaded before they are added: two with one row a warp, one with three rows (the registers
+// of two cost a third of the warps: 40x40x40 Hex8 255 us a step with one, 266 with two).  Where the call's
+// rows are all in flight at once anyway (FEW), the chain of a row's loads is the time: the warps get more
+// registers and load two incidences ahead (four for Tet4, whose rows are up to 24 cells long).  First K
+// of 17x18x15 Hex8 49.2 -> 39.6 us, 6x6x6 Tet4 33.6 -> 29.3, 6x6x6 Hex20 45.5 -> 39.7; four incidences for Hex8
+// or Hex20 gave the same as two.
+template <int NN, bool TRI, bool FEW>
+__global__ void __launch_bounds__(GATHER_WARPS * 32, FEW ? 2 : 3) gather3_kernel(GatherArgs P) {
     constexpr int NU = NN * (NN + 1) / 2;
     using GS = Gather3<NN>;
-    constexpr int ROWS = GS::ROWS, BPI = GS::BPI, NIT = GS::NIT, NB = GS::NB, CL = GS::CL;
+    constexpr int ROWS = GS::ROWS, BPI = GS::BPI, NIT = GS::NIT, CL = GS::CL;
+    constexpr int NB = ROWS == 1 ? 2 : !FEW ? 1 : NN > 4 ? 2 : 4;
     extern __shared__ double rowbuf[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     const int e = lane % 9, sub = lane / 9;  // lanes 27..31: sub = 3, no blocks
@@ -270,10 +277,12 @@ __global__ void __launch_bounds__(GATHER_WARPS * 32, 5) gather2_kernel(GatherArg
 }
 
 template <int ND, int NN>
-GatherShape shape_t(bool tri, int nbmax) {
+GatherShape shape_t(bool tri, bool few, int nbmax) {
     GatherShape s;
     if constexpr (ND == 3) {
-        s.kern = tri ? (const void*)gather3_kernel<NN, true> : (const void*)gather3_kernel<NN, false>;
+        s.kern = tri ? (const void*)gather3_kernel<NN, true, false> : (const void*)gather3_kernel<NN, false, false>;
+        if constexpr (Gather3<NN>::FEW)
+            if (few) s.kern = tri ? (const void*)gather3_kernel<NN, true, true> : (const void*)gather3_kernel<NN, false, true>;
         s.rows = Gather3<NN>::ROWS;
     } else {
         s.kern = tri ? (const void*)gather2_kernel<NN, true> : (const void*)gather2_kernel<NN, false>;
@@ -289,19 +298,19 @@ GatherShape shape_t(bool tri, int nbmax) {
 
 namespace pms {
 
-GatherShape gather_shape(int kind, bool triangle, int nbmax) {
+GatherShape gather_shape(int kind, bool triangle, bool few, int nbmax) {
     switch (kind) {
-    case PMS_TRI3: return shape_t<2, 3>(triangle, nbmax);
-    case PMS_TRI6: return shape_t<2, 6>(triangle, nbmax);
-    case PMS_QUA4: return shape_t<2, 4>(triangle, nbmax);
-    case PMS_QUA8: return shape_t<2, 8>(triangle, nbmax);
-    case PMS_QUA9: return shape_t<2, 9>(triangle, nbmax);
-    case PMS_TRI10: return shape_t<2, 10>(triangle, nbmax);
-    case PMS_TRI15: return shape_t<2, 15>(triangle, nbmax);
-    case PMS_TET4: return shape_t<3, 4>(triangle, nbmax);
-    case PMS_TET10: return shape_t<3, 10>(triangle, nbmax);
-    case PMS_HEX8: return shape_t<3, 8>(triangle, nbmax);
-    default: return shape_t<3, 20>(triangle, nbmax);
+    case PMS_TRI3: return shape_t<2, 3>(triangle, few, nbmax);
+    case PMS_TRI6: return shape_t<2, 6>(triangle, few, nbmax);
+    case PMS_QUA4: return shape_t<2, 4>(triangle, few, nbmax);
+    case PMS_QUA8: return shape_t<2, 8>(triangle, few, nbmax);
+    case PMS_QUA9: return shape_t<2, 9>(triangle, few, nbmax);
+    case PMS_TRI10: return shape_t<2, 10>(triangle, few, nbmax);
+    case PMS_TRI15: return shape_t<2, 15>(triangle, few, nbmax);
+    case PMS_TET4: return shape_t<3, 4>(triangle, few, nbmax);
+    case PMS_TET10: return shape_t<3, 10>(triangle, few, nbmax);
+    case PMS_HEX8: return shape_t<3, 8>(triangle, few, nbmax);
+    default: return shape_t<3, 20>(triangle, few, nbmax);
     }
 }
 

@@ -62,13 +62,14 @@ struct GatherArgs {
     const int64_t* tbase;
 };
 
-// Kernel and launch shape of an element kind's gather.
+// Kernel and launch shape of an element kind's gather; few: the kernel for calls whose rows are all in
+// flight at once, where the kind has one (Tet4, Hex8, Hex20).
 struct GatherShape {
     const void* kern;
     int rows;  // block rows per warp
     int wpb;   // warps per block
     int smem;  // bytes per block
 };
-GatherShape gather_shape(int kind, bool triangle, int nbmax);
+GatherShape gather_shape(int kind, bool triangle, bool few, int nbmax);
 
 }  // namespace pms

@@ -41,7 +41,7 @@ struct WorkQueue {
 };
 
 // One launch of the element kernel in per-problem mode (0 skip, 1 step start, 2 update) followed by
-// the F_int and CSR gathers (the CSR rows of mode-0 problems are left as they are); all pointers
+// the gather of K and R (the CSR rows of mode-0 problems are left as they are); all pointers
 // are device pointers on the handle's stream.  With a queue, only its cells and nodes are visited
 // (every queued problem must have a non-zero mode); F_int rows outside the queue are left as they are.
 // prob_err (device, nullable): per problem, the key of the element error that problem would report

@@ -365,3 +365,32 @@ def test_host_arrays_pageable_pinned_and_device(kind, n):
             ff = np.zeros(g.ndof)
             g.update_and_assemble(ddu, ff, kv)
             assert np.array_equal(kv, d_kv.cpu().numpy()) and np.array_equal(ff, d_ff.cpu().numpy())
+
+
+@pytest.mark.parametrize("kind,ngauss,n", [(M.TET4, 4, (2, 2, 2)), (M.TET4, 4, (7, 6, 5)), (M.HEX8, 8, (2, 2, 2)),
+                                           (M.HEX8, 8, (9, 8, 7)), (M.HEX8, 8, (19, 18, 18)),
+                                           (M.HEX20, 8, (3, 2, 2)), (M.HEX20, 8, (6, 6, 6))])
+@pytest.mark.parametrize("sym", ["full", "lower"])
+def test_gather_of_few_rows(kind, ngauss, n, sym):
+    """The gather loads further ahead where all rows are in flight at once: rows of one cell and of many,
+    numbers of cells that are no multiple of the cells loaded together, and a mesh past the line, against
+    the oracle at the parity tolerance."""
+    from pmsim_b200.elements import Elements, Material
+    m = perturbed_mesh(kind, seed=5, n=n)
+    g = Elements(m, Material.von_mises(E, NU, H, Z0), ngauss=ngauss)
+    o = oracle.OracleElements(m, 1, oracle.Params(E, NU, H, Z0), ngauss=ngauss, sym_tol=-1.0, nthreads=0)
+    indptr, indices = g.csr_pattern()
+    ddu = plastic_ddu(m, seed=6)
+    g.initialize_internal_values()
+    o.initialize()
+    g.backup_secondary_values()
+    g.set_symmetry(sym)
+    ff, kv = np.zeros(g.ndof), np.zeros(g.nnz)
+    g.update_and_assemble(ddu, ff, kv)
+    o.update_secondary_values(ddu)
+    ko = oracle_csr_values(o, indptr, indices)
+    if sym == "lower":
+        rows = np.repeat(np.arange(len(indptr) - 1), np.diff(indptr))
+        ko = ko[np.asarray(indices) <= rows]
+    assert_close(ff, o.assemble_f_int(), what="f_int")
+    assert_close(kv, ko, what="K")
