@@ -376,8 +376,8 @@ def run_qua8_step(torch, stream, steps, warmup, hbm_peak, n=1024):
     gbs_step = step_bytes / (ms * 1e-3) / 1e9
     return {"workload": f"qua8 {n}x{n} footing material, 9 IP, one fused Newton iteration", "ncell": m.ncell,
             "nip": nip, "nnz": int(el.nnz), "plastic_fraction": plastic, "ms_per_step": ms,
-            "kernels": "element2d_kernel<8,10,UPD_BACKUP,F,K> (update + F_int + upper K_e blocks), f_gather, "
-                       "kk_gather<2,8> (rows summed in ascending cell order)",
+            "kernels": "element2d_kernel<8,10,UPD_BACKUP,F,K> (update + F_int + upper K_e blocks), "
+                       "gather2_kernel<8> (rows of K and R summed in ascending cell order)",
             "kernels_ms_per_step": kernel_ms(kt, kc),
             "assembly_ab": ab,
             "step_roofline": {"bound": "hbm", "achieved": gbs_step, "peak": hbm_peak, "unit": "GB/s",
@@ -444,7 +444,8 @@ def lower_triangle_step(torch, L, el, stream, steps, warmup, d_ddu, d_ff):
 
 
 def kernel_ms(kt, kc):
-    """Per-step times of the element kernel and the two gathers (absent under the direct assembly)."""
+    """Per-step times of the element kernel and of the gathers (absent under the direct assembly; the
+    gather of K forms R as well, so f_gather appears only for calls without K)."""
     out = {"element": kt[0] / max(kc[0], 1)}
     if kc[1]:
         out["f_gather"] = kt[1] / kc[1]
