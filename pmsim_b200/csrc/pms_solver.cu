@@ -1450,7 +1450,9 @@ WideShape wide_shape(const pms_batch* b) {
     return s;
 }
 
-WideArgs wide_args(const pms_batch* b, int budget, int stop) {
+// budget: any non-negative count; the kernel gets the next even one that its 32-bit counter holds, so that a
+// cap of "no limit" (up to INT32_MAX iterations) stays one.
+WideArgs wide_args(const pms_batch* b, int64_t budget, int stop) {
     WideArgs w;
     w.quarter = b->d_quarter;
     w.bcol = b->v.d_bcol;
@@ -1471,14 +1473,14 @@ WideArgs wide_args(const pms_batch* b, int budget, int stop) {
     w.ctl = b->d_ctl;
     w.rtol = b->cfg.pcg_rtol;
     w.max_iter = b->cfg.pcg_max_iterations;
-    w.budget = (budget + 1) & ~1;
+    w.budget = (int32_t)std::min<int64_t>((budget + 1) & ~int64_t(1), INT32_MAX - 1);
     w.stop = stop;
     return w;
 }
 
 // Up to `budget` iterations of the active problems on the batch-wide engine; it ends early, at an even
 // iteration, once `stop` problems have finished.
-int launch_wide(pms_batch* b, int budget, int stop, cudaStream_t st) {
+int launch_wide(pms_batch* b, int64_t budget, int stop, cudaStream_t st) {
     const WideShape s = wide_shape(b);
     WideArgs w = wide_args(b, budget, stop);
     int maxruns = s.maxruns, maxshare = s.maxshare;
@@ -2279,7 +2281,7 @@ int build_step_graph(pms_batch* b) {
     if (coop) {
         // the PCG of every problem to its end
         const WideShape wshape = wide_shape(b);
-        WideArgs wargs = wide_args(b, b->cfg.pcg_max_iterations + 2, INT32_MAX);
+        WideArgs wargs = wide_args(b, (int64_t)b->cfg.pcg_max_iterations + 2, INT32_MAX);
         int wruns = wshape.maxruns, wshare = wshape.maxshare;
         void* a_pcg[] = {&S, &wargs, &wruns, &wshare};
         body.zero(b->d_ctl, 2);  // the failure flag stays for the host

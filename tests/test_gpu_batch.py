@@ -291,3 +291,25 @@ def test_batch_wide_engines_give_the_same_bits(nx, count):
         for x, y in zip(out[0][:4], o[:4]):
             assert np.array_equal(x, y)
         assert out[0][4:] == o[4:]
+
+
+@pytest.mark.parametrize("cap", [1, 7, 2 ** 31 - 4, 2 ** 31 - 3, 2 ** 31 - 2, 2 ** 31 - 1])
+def test_pcg_iteration_caps_up_to_the_largest(cap):
+    """pcg_max_iterations from one iteration to the largest value its type holds (no cap): the batch-wide
+    engine, host-sequenced and in the device-resident load step, gives the iterates, the iteration
+    counts and the failures of the teams."""
+    from pmsim_b200.batch import BatchSolver
+    probs = [footing(9 + 3 * i, 5 + i, 1e4 * (1 + 0.2 * i), 9.0 + i, 1.0, nsteps=2) for i in range(3)]
+    out = []
+    for mode in ("teams", "wide", "device"):
+        b = BatchSolver(probs, pcg_max_iterations=cap)
+        if mode == "wide":
+            b.set_tuning(**{**b.tuning(), "team_max_ndof": 0})
+        b.solve(device_loop=mode == "device", on_fail="drop")
+        out.append((b.u(), *b.elements.get_state(), b.history, b.pcg_history, b.failed))
+    for o in out[1:]:
+        for x, y in zip(out[0][:4], o[:4]):
+            assert np.array_equal(x, y)
+        assert out[0][4:] == o[4:]
+    if cap > 1000:
+        assert not out[0][6] and all(n > 0 for h in out[0][5] for n in h)
