@@ -1614,11 +1614,12 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
 }
 
 // R alone (no K asked for): one thread per point, R[A*nd + i] = sum over its incidences (ascending cell)
-// of f_e.
+// of f_e.  fe is not __restrict__: it may be written while this kernel, launched early, waits, and so must
+// not go through the read-only path.
 template <int ND>
 __global__ void __launch_bounds__(256) f_gather_kernel(int64_t npoint, const int64_t* __restrict__ inc_ptr,
                                                        const int32_t* __restrict__ inc,
-                                                       const double* __restrict__ fe, double* __restrict__ ff) {
+                                                       const double* fe, double* ff) {
     let_next_start();
     wait_for_previous();
     for (int64_t A = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; A < npoint;

@@ -14,7 +14,9 @@ constexpr unsigned FULL = 0xffffffffu;
 // read transposed where b < a -- at column slot[k*NN + b] of the row's buffer in shared memory, and
 // writes the row once, coalesced.  The incidences go in ascending (= cell) order, so every entry of
 // K is the fixed-order sum over its cells: bit-identical on every run.  The same pass forms R (row A
-// sums its cells' F_e).
+// sums its cells' F_e).  ke and fe are read by ordinary loads: a launch that overlaps the element kernel
+// is resident while they are written, and the read-only path (__ldg) is for memory that stays as it is from
+// the kernel's start to its end; the maps of the mesh do.
 //
 // Bounds: 64x64x32 Hex20 moves 4.2 GB (0.65 ms at 6.5 TB/s) and takes 1.57 ms, as before with a lane per
 // 3x3 block: the LSU data pipe (each 8-byte value is loaded, added in shared memory and written out)
@@ -119,13 +121,13 @@ __global__ void __launch_bounds__(GATHER_WARPS * 32, FEW ? 2 : 3) gather3_kernel
                 const double* up = kc + 9 * (upper_block(NN, a, a) - a) + e;
                 const double* lo = kc + 9 * a + et;
                 const int16_t* sl = P.slot + (k0 + n) * NN;
-                fv[t] = (acc_f && on) ? __ldg(P.fe + (int64_t)cd * 3 + e) : 0.0;
+                fv[t] = (acc_f && on) ? P.fe[(int64_t)cd * 3 + e] : 0.0;
 #pragma unroll
                 for (int u = 0; u < NIT; u++) {
                     const int b = u * BPI + b0;
                     const bool have = on && (NIT * BPI == NN || b < NN);
                     pos[t][u] = have ? (int)__ldg(sl + b) : -1;
-                    v[t][u] = have ? __ldg(b >= a ? up + 9 * b : lo + 9 * (upper_block(NN, b, b) - b)) : 0.0;
+                    v[t][u] = have ? *(b >= a ? up + 9 * b : lo + 9 * (upper_block(NN, b, b) - b)) : 0.0;
                 }
             }
             if (!zeroed) {  // while the first loads are under way
@@ -230,10 +232,10 @@ __global__ void __launch_bounds__(GATHER_WARPS * 32, 5) gather2_kernel(GatherArg
                 const bool upper = a <= b;
                 const double2* src = reinterpret_cast<const double2*>(
                     P.ke + 4 * ((int64_t)cell * NU + upper_block(NN, upper ? a : b, upper ? b : a)));
-                u = __ldg(src);
-                v = __ldg(src + 1);
+                u = src[0];
+                v = src[1];
                 pos = __ldg(P.slot + (k0 + n) * NN + b);
-                if (acc_f) fv = __ldg(P.fe + (int64_t)cd * 2 + b);
+                if (acc_f) fv = P.fe[(int64_t)cd * 2 + b];
                 if (!upper) {
                     const double x = u.y;
                     u.y = v.x;

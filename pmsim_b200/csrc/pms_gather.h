@@ -9,8 +9,8 @@ namespace pms {
 
 // Programmatic dependent launch: the kernels of a batched call (element kernel, then gather) let the
 // next one's blocks start as soon as their own have, and wait for the previous kernel to finish
-// before they touch its results, so that launch and start-up overlap its end.  Both are no-ops after
-// an ordinary launch.  Only where the gather is one wave (launch_overlapped's `overlap`): 20x10 Qua8
+// before they touch its results, so that launch and start-up overlap its end.  What they read of them
+// they read by ordinary loads (no __ldg, no const __restrict__).  Both are no-ops after an ordinary launch.  Only where the gather is one wave (launch_overlapped's `overlap`): 20x10 Qua8
 // step 16.4 -> 11.6 us, 87x48 Qua9 23.8 -> 20.1, 12x10x6 Hex20 51 -> 45; on larger meshes the early gather
 // blocks run at the element kernel's shared-memory carveout, where they miss in L1 (701x350 Qua8 526 ->
 // 864 us).

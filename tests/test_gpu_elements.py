@@ -394,3 +394,39 @@ def test_gather_of_few_rows(kind, ngauss, n, sym):
         ko = ko[np.asarray(indices) <= rows]
     assert_close(ff, o.assemble_f_int(), what="f_int")
     assert_close(kv, ko, what="K")
+
+
+@pytest.mark.parametrize("kind,ngauss,n", [(M.QUA8, 9, (20, 10, 1)), (M.TRI6, 3, (9, 8, 1)), (M.TET4, 4, (4, 3, 3)),
+                                           (M.HEX8, 8, (6, 5, 5)), (M.HEX20, 27, (3, 3, 2))],
+                         ids=["qua8", "tri6", "tet4", "hex8", "hex20"])
+def test_calls_that_follow_one_another_without_a_wait(kind, ngauss, n):
+    """On small meshes the kernels of successive calls overlap their launches while the element matrices are
+    written again and again: K and R of many calls in a row, each with another increment (and F_int alone
+    in between), are the bits of the same calls made one at a time."""
+    import torch
+    from pmsim_b200.elements import Elements, Material
+    m = perturbed_mesh(kind, seed=8, n=n)
+    g = Elements(m, Material.von_mises(E, NU, H, Z0), ngauss=ngauss)
+    g.initialize_internal_values()
+    g.backup_secondary_values()
+    count = 60
+    ddu = [torch.tensor(plastic_ddu(m, seed=10 + k) * (0.2 + 0.05 * k), device="cuda") for k in range(count)]
+    runs = []
+    for wait in (True, False):
+        ff = torch.zeros(count, g.ndof, dtype=torch.float64, device="cuda")
+        f2 = torch.zeros(count, g.ndof, dtype=torch.float64, device="cuda")
+        kk = torch.zeros(count, g.nnz, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        for k in range(count):
+            g.update_and_assemble(ddu[k], ff[k], kk[k])
+            if wait:
+                g.sync()
+            if k % 3 == 2:
+                g.assemble_f_int(f2[k])
+                if wait:
+                    g.sync()
+        g.sync()
+        runs.append((ff.cpu().numpy(), f2.cpu().numpy(), kk.cpu().numpy()))
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
+    assert not np.array_equal(runs[0][2][0], runs[0][2][-1])  # (the first increments are elastic)
