@@ -40,6 +40,7 @@
 #include "../../include/pms.h"
 #include "pms_device.cuh"
 #include "pms_internal.h"
+#include "pms_per_device.h"
 
 using namespace pms;
 
@@ -1535,21 +1536,22 @@ bool team_attrs_t() {
                cudaSuccess;
 }
 
-// Kernel attributes of every team variant, and the largest cluster this device schedules
-// (16 where the non-portable size is available, else 8).  Once per process.
+// Kernel attributes of every team variant on the current device, and the largest cluster it schedules
+// (16 where the non-portable size is available, else 8).  An attribute holds for the device it was set on, so
+// this is done once on each.
 int team_setup(int* cmax) {
-    static int cached = -1;
-    static std::mutex m;
-    std::lock_guard<std::mutex> lock(m);
-    if (cached < 0) {
-        const bool ok = team_attrs_t<256, 8>() && team_attrs_t<256, 16>() && team_attrs_t<512, 8>() &&
-                        team_attrs_t<512, 16>() && team_attrs_t<1024, 8>() && team_attrs_t<1024, 16>() &&
-                        cudaFuncSetAttribute(pcg_wide_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)TEAM_SMEM_LIMIT) == cudaSuccess &&
-                        cudaFuncSetAttribute(pcg_wide_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)TEAM_SMEM_LIMIT) == cudaSuccess;
-        if (!ok) return PMS_ERR_CUDA;
-        int c = 16;
+    static PerDevice<int> known;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const bool ok = known.get(dev, *cmax, [](int& c) {
+        if (!(team_attrs_t<256, 8>() && team_attrs_t<256, 16>() && team_attrs_t<512, 8>() &&
+              team_attrs_t<512, 16>() && team_attrs_t<1024, 8>() && team_attrs_t<1024, 16>() &&
+              cudaFuncSetAttribute(pcg_wide_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)TEAM_SMEM_LIMIT) == cudaSuccess &&
+              cudaFuncSetAttribute(pcg_wide_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)TEAM_SMEM_LIMIT) == cudaSuccess))
+            return false;
+        c = 16;
         for (int nd = 2; nd <= 3; nd++) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(16);
@@ -1568,10 +1570,9 @@ int team_setup(int* cmax) {
             if (e != cudaSuccess) cudaGetLastError();
             if (e != cudaSuccess || n16 < 1) c = 8;
         }
-        cached = c;
-    }
-    *cmax = cached;
-    return PMS_OK;
+        return true;
+    });
+    return ok ? PMS_OK : PMS_ERR_CUDA;
 }
 
 // Team size of a problem: the smallest power of two whose CTAs hold at most the target number of
@@ -1670,50 +1671,44 @@ int pcg_phase(pms_batch* b, int nteam, int nwide, int budget, bool exact) {
 }
 
 // Teams of each size that the device holds at once, at the launch shape a batch starts with (looked up
-// once per device and dimension: the queries take 2 to 4 ms).
+// once per device and dimension: the queries take 2 to 4 ms).  Where they fail the teams stay as tuned.
 void count_team_slots(pms_batch* b) {
-    constexpr int MAXDEV = 64;
-    static std::mutex m;
-    static int known[MAXDEV][2][NCLASS];
-    static bool have[MAXDEV][2];
+    struct Slots {
+        int n[NCLASS];
+    };
+    static PerDevice<Slots> known[2];
     int dev = 0;
     cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(m);
-    const int dim = b->v.nd == 2 ? 0 : 1;
-    if (dev < MAXDEV && have[dev][dim]) {
-        std::copy(known[dev][dim], known[dev][dim] + NCLASS, b->team_slots);
-        return;
-    }
     const bool two = tpr_of(b->v.nd) == 8;
-    const void* kern = nullptr;
-    switch (b->tune.team_threads) {
-        case 256: kern = two ? (const void*)pcg_team_kernel<256, 8> : (const void*)pcg_team_kernel<256, 16>; break;
-        case 1024: kern = two ? (const void*)pcg_team_kernel<1024, 8> : (const void*)pcg_team_kernel<1024, 16>; break;
-        default: kern = two ? (const void*)pcg_team_kernel<512, 8> : (const void*)pcg_team_kernel<512, 16>; break;
-    }
-    for (int c = 0; c < NCLASS; c++) {
-        b->team_slots[c] = 0;
-        if ((1 << c) > b->team_cmax) continue;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(1u << c);
-        cfg.blockDim = dim3((unsigned)b->tune.team_threads);
-        cfg.dynamicSmemBytes = team_smem_bytes(b->v.nd, b->tune.team_threads);
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 1u << c;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&b->team_slots[c], kern, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            b->team_slots[c] = 0;
+    Slots s{};
+    const bool ok = known[two ? 0 : 1].get(dev, s, [&](Slots& r) {
+        const void* kern = nullptr;
+        switch (b->tune.team_threads) {
+            case 256: kern = two ? (const void*)pcg_team_kernel<256, 8> : (const void*)pcg_team_kernel<256, 16>; break;
+            case 1024: kern = two ? (const void*)pcg_team_kernel<1024, 8> : (const void*)pcg_team_kernel<1024, 16>; break;
+            default: kern = two ? (const void*)pcg_team_kernel<512, 8> : (const void*)pcg_team_kernel<512, 16>; break;
         }
-    }
-    if (dev < MAXDEV) {
-        std::copy(b->team_slots, b->team_slots + NCLASS, known[dev][dim]);
-        have[dev][dim] = true;
-    }
+        for (int c = 0; c < NCLASS && (1 << c) <= b->team_cmax; c++) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(1u << c);
+            cfg.blockDim = dim3((unsigned)b->tune.team_threads);
+            cfg.dynamicSmemBytes = team_smem_bytes(b->v.nd, b->tune.team_threads);
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = 1u << c;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&r.n[c], kern, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+        }
+        return true;
+    });
+    std::copy(s.n, s.n + NCLASS, b->team_slots);
+    if (!ok) b->fit_teams = false;
 }
 
 // Team size (as its power of two) of a problem of nch chunks at `per` chunks per CTA; -1: too large.

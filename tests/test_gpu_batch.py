@@ -313,3 +313,29 @@ def test_pcg_iteration_caps_up_to_the_largest(cap):
         assert out[0][4:] == o[4:]
     if cap > 1000:
         assert not out[0][6] and all(n > 0 for h in out[0][5] for n in h)
+
+
+def test_batches_on_each_device():
+    """A batch on every GPU of the machine, made by a thread of its own as the server does it, with clusters
+    whose shared memory needs the kernel attributes set on that device: the same bits."""
+    import threading
+    import torch
+    from pmsim_b200 import _lib
+    from pmsim_b200.batch import BatchSolver
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one GPU")
+    probs = [footing(10 + i, 5 + i, 1e4, 9.0 + i, 1.0, nsteps=1) for i in range(4)]
+    out = {}
+
+    def work(dev):
+        _lib.set_device(dev)
+        b = BatchSolver(probs)
+        iters = b.solve_step()[0]
+        out[dev] = (b.u(), iters)
+        b.close()
+
+    for dev in range(2):
+        th = threading.Thread(target=work, args=(dev,))
+        th.start()
+        th.join()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
