@@ -1728,6 +1728,7 @@ struct pms_elements {
     int32_t* d_indices = nullptr;
     int32_t* d_status = nullptr;
     int64_t device_bytes = 0;
+    int device = 0;  // its memory and its own stream are there
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
     std::string last_error;
@@ -1815,6 +1816,21 @@ int cuda_check(pms_elements* h) {
     if (e != cudaSuccess) return fail(h, PMS_ERR_CUDA, cudaGetErrorString(e));
     return PMS_OK;
 }
+
+// Makes the handle's device current for a call that may be made while another one is.
+struct OnDevice {
+    int before = 0;
+    explicit OnDevice(const pms_elements* h) {
+        cudaGetDevice(&before);
+        if (before != h->device) cudaSetDevice(h->device);
+        else before = -1;
+    }
+    ~OnDevice() {
+        if (before >= 0) cudaSetDevice(before);
+    }
+    OnDevice(const OnDevice&) = delete;
+    OnDevice& operator=(const OnDevice&) = delete;
+};
 
 int grid_1d(int64_t n) {
     int64_t b = (n + 255) / 256;
@@ -2134,6 +2150,7 @@ int pms_elements_create(const pms_mesh* mesh, const pms_material* materials, int
                 return refuse(PMS_ERR_INVALID, "cell_material names a material that does not exist");
     }
     auto* h = new pms_elements();
+    cudaGetDevice(&h->device);
     h->kind = kind;
     h->nd = mesh->ndim;
     h->nc = 2 * h->nd;
@@ -2597,7 +2614,9 @@ int pms_element_calc_jacobian(pms_elements* h, int64_t cell, double* kk) {
 
 int pms_elements_get_state(pms_elements* h, double* sig, double* ivs, uint8_t* elastic) {
     if (!h) return PMS_ERR_INVALID;
-    // ordered by IP on the device, in pieces of the scratch, then straight to the caller's arrays
+    // ordered by IP on the device, in pieces of the scratch, then straight to the caller's arrays.  The state may
+    // be read while another device is current, so the scratch and the kernel are placed by the handle
+    const OnDevice on(h);
     const int64_t n = h->nip, per = h->nc + 2;
     double* d = h->d_pack;
     int64_t room = h->pack_ips;

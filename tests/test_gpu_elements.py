@@ -430,3 +430,37 @@ def test_calls_that_follow_one_another_without_a_wait(kind, ngauss, n):
     for a, b in zip(*runs):
         assert np.array_equal(a, b)
     assert not np.array_equal(runs[0][2][0], runs[0][2][-1])  # (the first increments are elastic)
+
+
+def test_state_is_read_while_another_device_is_current():
+    """get_state needs no particular current device, leaves the one it finds current, and gives what it gives
+    on the handle's own."""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one GPU")
+    m, g, _ = make(M.HEX8, seed=9)
+    g.initialize_internal_values()
+    g.update_secondary_values(plastic_ddu(m, seed=10))
+    g.sync()
+    with torch.cuda.device(1):
+        first = g.get_state()  # (its scratch is made here)
+        again = g.get_state()
+        assert torch.cuda.current_device() == 1
+        torch.zeros(1, device="cuda").add_(1.0)
+    for a, b, c in zip(first, again, g.get_state()):
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+
+
+@pytest.mark.parametrize("want", [(1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1), (0, 0, 0)])
+def test_state_arrays_are_optional(want):
+    """Any of the three arrays of pms_elements_get_state may be null; the others are the same."""
+    from pmsim_b200 import _lib
+    m, g, _ = make(M.QUA8, seed=9)
+    g.initialize_internal_values()
+    g.update_secondary_values(plastic_ddu(m, seed=10))
+    full = g.get_state()
+    arrays = [np.full_like(a, 7) for a in full]
+    rc = g.L.pms_elements_get_state(g.h, *(_lib.ptr(a) if w else None for a, w in zip(arrays, want)))
+    assert rc == 0
+    for a, f, w in zip(arrays, full, want):
+        assert np.array_equal(a, f if w else np.full_like(f, 7))
