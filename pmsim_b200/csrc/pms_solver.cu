@@ -1278,9 +1278,10 @@ struct pms_batch {
     double *d_part_a = nullptr, *d_part_b = nullptr, *d_part_c = nullptr;
     double *d_rho = nullptr, *d_r0 = nullptr, *d_norm = nullptr, *d_rel = nullptr;
     int32_t *d_iters = nullptr, *d_nactive = nullptr;
-    double *d_p1 = nullptr, *d_part_q = nullptr;  // batch-wide engine: second direction, r.z and r.r quarters
-    unsigned* d_ctl = nullptr;                    // its barrier, finished problems, failure flag
-    WideQuarter* d_quarter = nullptr;             // its units of work
+    // cooperative batch-wide engine (wide_in_one_kernel)
+    double *d_p1 = nullptr, *d_part_q = nullptr;  // second direction, r.z and r.r quarters
+    unsigned* d_ctl = nullptr;                    // barrier, finished problems, failure flag (every batch)
+    WideQuarter* d_quarter = nullptr;             // units of work
     int64_t* d_queue = nullptr;    // work queue of the element pass: 4 arrays of np + 1
     unsigned long long* d_perr = nullptr;  // per problem: key of its element error in the last pass
     // device-resident load step
@@ -1424,6 +1425,9 @@ int ensure_graph(pms_batch* b) {
     b->graph_iters_captured = gi;
     return PMS_OK;
 }
+
+// Which form of the batch-wide engine a batch takes (the cooperative kernel's buffers exist only then).
+bool wide_in_one_kernel(const pms_batch* b) { return b->nchunk <= WIDE_MAX_CHUNKS; }
 
 // Launch shape and arguments of the cooperative batch-wide engine.  grid: as many blocks as the device holds, at most
 // one per group of quarters worked on together.
@@ -1634,7 +1638,7 @@ int pcg_phase(pms_batch* b, int nteam, int nwide, int budget, bool exact) {
     };
     if (nwide > 0) {
         // cooperative: eight times the graph_iters of the tuning per launch and wait of the host
-        const bool coop = b->nchunk <= WIDE_MAX_CHUNKS;
+        const bool coop = wide_in_one_kernel(b);
         if (!coop) {
             int rc = ensure_graph(b);
             if (rc) return rc;
@@ -1873,8 +1877,9 @@ int pms_batch_create(pms_elements* el, int32_t nproblem, const int64_t* point_pt
               b->alloc(&b->d_rho, 2 * (size_t)nproblem) && b->alloc(&b->d_r0, nproblem) &&
               b->alloc(&b->d_norm, nproblem) && b->alloc(&b->d_rel, nproblem) &&
               b->alloc(&b->d_iters, 2 * (size_t)nproblem) &&
-              b->alloc(&b->d_nactive, 1) && b->alloc(&b->d_p1, n) && b->alloc(&b->d_part_q, 8 * (size_t)b->nchunk) && b->alloc(&b->d_ctl, 4) &&
-              b->alloc(&b->d_quarter, 4 * (size_t)b->nchunk) &&
+              b->alloc(&b->d_nactive, 1) && b->alloc(&b->d_ctl, 4) &&
+              (!wide_in_one_kernel(b) || (b->alloc(&b->d_p1, n) && b->alloc(&b->d_part_q, 8 * (size_t)b->nchunk) &&
+                                          b->alloc(&b->d_quarter, 4 * (size_t)b->nchunk))) &&
               b->alloc(&b->d_queue, 4 * ((size_t)nproblem + 1)) &&
               b->alloc(&b->d_perr, (size_t)nproblem) && b->alloc(&b->d_phase, nproblem) &&
               b->alloc(&b->d_sel, nproblem) && b->alloc(&b->d_zero_engine, nproblem) &&
@@ -1925,8 +1930,9 @@ int pms_batch_create(pms_elements* el, int32_t nproblem, const int64_t* point_pt
     b->pnch.assign(nproblem, 0);
     for (int p = 0; p < nproblem; p++) b->pnch[p] = pchunk[p + 1] - pchunk[p];
     count_team_slots(b);
-    wide_quarters_kernel<<<grid_of(32 * 4 * b->nchunk), 256>>>(4 * b->nchunk, b->d_chunk_node0, b->d_chunk_nnode,
-                                                                b->v.d_bptr, b->d_quarter);
+    if (wide_in_one_kernel(b))
+        wide_quarters_kernel<<<grid_of(32 * 4 * b->nchunk), 256>>>(4 * b->nchunk, b->d_chunk_node0, b->d_chunk_nnode,
+                                                                    b->v.d_bptr, b->d_quarter);
     if (assign_engines(b) || cudaDeviceSynchronize() != cudaSuccess) {
         delete b;
         return PMS_ERR_CUDA;
@@ -2220,7 +2226,7 @@ int build_step_graph(pms_batch* b) {
     S.engine = b->d_zero_engine;  // every PCG on the batch-wide engine (the engines give the same bits)
     double tol_rr = b->cfg.tol_rr_abs, tol_mdu = b->cfg.tol_mdu_rel, rtol = b->cfg.pcg_rtol;
     int32_t max_it = b->cfg.n_max_iterations, max_pcg = b->cfg.pcg_max_iterations;
-    const bool coop = b->nchunk <= WIDE_MAX_CHUNKS;
+    const bool coop = wide_in_one_kernel(b);
     int use_loop = coop ? 0 : 1;
     int zero = 0;
     bool no_mask = false;
