@@ -2812,9 +2812,8 @@ int elements_device_pattern(pms_elements* h, const int64_t** indptr, const int32
     return PMS_OK;
 }
 
-int elements_run_modes(pms_elements* h, const int32_t* cell_prob, const int32_t* node_prob, const uint8_t* pmode,
-                       const double* ddu, double* ff, double* csr, const WorkQueue* queue,
-                       unsigned long long* prob_err) {
+int elements_run_modes(pms_elements* h, const int32_t* cell_prob, const uint8_t* pmode, const double* ddu, double* ff,
+                       double* csr, const WorkQueue* queue, unsigned long long* prob_err) {
     ElemArgs a = make_args(h, ddu);
     a.cell_prob = cell_prob;
     a.pmode = pmode;
@@ -2828,7 +2827,6 @@ int elements_run_modes(pms_elements* h, const int32_t* cell_prob, const int32_t*
     }
     a.csr = csr;  // direct assembly: rows of problems outside the pass are left as they are
     a.ff = ff;
-    (void)node_prob;
     launch_elem(h, a, UPD_MODE, true, true, true);
     return cuda_check(h);
 }

@@ -29,26 +29,23 @@ ElementsView elements_view(pms_elements* h);
 // Device CSR pattern of K (allocated by the handle on first use, kept until destroy).
 int elements_device_pattern(pms_elements* h, const int64_t** indptr, const int32_t** indices);
 
-// Work queue of a batched element pass: the cell ranges and node ranges of the problems that take
-// part (device arrays; range k covers off[k] .. off[k+1]-1 of the queue, starting at first[k]).
+// Work queue of a batched element pass: the cell ranges of the problems that take part (device arrays;
+// range k covers off[k] .. off[k+1]-1 of the queue, starting at first[k]).
 struct WorkQueue {
     int32_t nq = 0;
-    int64_t ncell = 0, nnode = 0;  // queued cells and nodes (off[nq])
+    int64_t ncell = 0;  // queued cells (off[nq])
     const int64_t* cell_off = nullptr;
     const int64_t* cell_first = nullptr;
-    const int64_t* node_off = nullptr;
-    const int64_t* node_first = nullptr;
 };
 
-// One launch of the element kernel in per-problem mode (0 skip, 1 step start, 2 update) followed by
-// the gather of K and R (the CSR rows of mode-0 problems are left as they are); all pointers
-// are device pointers on the handle's stream.  With a queue, only its cells and nodes are visited
-// (every queued problem must have a non-zero mode); F_int rows outside the queue are left as they are.
+// One launch of the element kernel in per-problem mode (0 skip, 1 step start, 2 update, 3 update with K kept),
+// which adds K and R itself (direct assembly; the rows of problems that do not take part are left as they are);
+// all pointers are device pointers on the handle's stream.  With a queue, only its cells are visited
+// (every queued problem must have a non-zero mode).
 // prob_err (device, nullable): per problem, the key of the element error that problem would report
 // (atomicMax; the caller zeroes it before the launch; decode with decode_error).
-int elements_run_modes(pms_elements* h, const int32_t* cell_prob, const int32_t* node_prob, const uint8_t* pmode,
-                       const double* ddu, double* ff, double* csr, const WorkQueue* queue = nullptr,
-                       unsigned long long* prob_err = nullptr);
+int elements_run_modes(pms_elements* h, const int32_t* cell_prob, const uint8_t* pmode, const double* ddu, double* ff,
+                       double* csr, const WorkQueue* queue = nullptr, unsigned long long* prob_err = nullptr);
 
 // Adds to graph g (after dep, if not null) a memset node that zeroes the element pass's in-order work
 // counter and the node of the per-problem-mode element kernel over every cell (direct assembly into

@@ -1282,7 +1282,7 @@ struct pms_batch {
     double *d_p1 = nullptr, *d_part_q = nullptr;  // second direction, r.z and r.r quarters
     unsigned* d_ctl = nullptr;                    // barrier, finished problems, failure flag (every batch)
     WideQuarter* d_quarter = nullptr;             // units of work
-    int64_t* d_queue = nullptr;    // work queue of the element pass: 4 arrays of np + 1
+    int64_t* d_queue = nullptr;    // work queue of the element pass: 2 arrays of np + 1
     unsigned long long* d_perr = nullptr;  // per problem: key of its element error in the last pass
     // device-resident load step
     cudaGraphExec_t step_graph = nullptr;
@@ -1880,7 +1880,7 @@ int pms_batch_create(pms_elements* el, int32_t nproblem, const int64_t* point_pt
               b->alloc(&b->d_nactive, 1) && b->alloc(&b->d_ctl, 4) &&
               (!wide_in_one_kernel(b) || (b->alloc(&b->d_p1, n) && b->alloc(&b->d_part_q, 8 * (size_t)b->nchunk) &&
                                           b->alloc(&b->d_quarter, 4 * (size_t)b->nchunk))) &&
-              b->alloc(&b->d_queue, 4 * ((size_t)nproblem + 1)) &&
+              b->alloc(&b->d_queue, 2 * ((size_t)nproblem + 1)) &&
               b->alloc(&b->d_perr, (size_t)nproblem) && b->alloc(&b->d_phase, nproblem) &&
               b->alloc(&b->d_sel, nproblem) && b->alloc(&b->d_zero_engine, nproblem) &&
               b->alloc(&b->d_st, nproblem) && b->alloc(&b->d_cnt, nproblem) && b->alloc(&b->d_pcgsum, nproblem) &&
@@ -1987,28 +1987,22 @@ int pms_batch_tick(pms_batch* b, const uint8_t* cmd, const double* c_values, int
         cudaMemcpyAsync(b->d_upd, start.data(), np, cudaMemcpyHostToDevice, st);
         zero_masked_kernel<<<grid_of(b->ndof), 256, 0, st>>>(b->S, b->d_upd, b->d_ddu);  // new step: dU = 0
         cudaMemcpyAsync(b->d_pmode, mode.data(), np, cudaMemcpyHostToDevice, st);
-        // work queue: the cell and node ranges of these problems only
+        // work queue: the cell ranges of these problems only
         const size_t W = (size_t)np + 1;
-        b->h_queue.assign(4 * W, 0);
+        b->h_queue.assign(2 * W, 0);
         WorkQueue q;
         for (int p = 0; p < np; p++) {
             if (!elem[p]) continue;
             const int k = q.nq++;
             b->h_queue[k + 1] = b->h_queue[k] + (b->cell_ptr[p + 1] - b->cell_ptr[p]);
             b->h_queue[W + k] = b->cell_ptr[p];
-            b->h_queue[2 * W + k + 1] = b->h_queue[2 * W + k] + (b->point_ptr[p + 1] - b->point_ptr[p]);
-            b->h_queue[3 * W + k] = b->point_ptr[p];
         }
         q.ncell = b->h_queue[q.nq];
-        q.nnode = b->h_queue[2 * W + q.nq];
         q.cell_off = b->d_queue;
         q.cell_first = b->d_queue + W;
-        q.node_off = b->d_queue + 2 * W;
-        q.node_first = b->d_queue + 3 * W;
-        cudaMemcpyAsync(b->d_queue, b->h_queue.data(), 4 * W * 8, cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(b->d_queue, b->h_queue.data(), 2 * W * 8, cudaMemcpyHostToDevice, st);
         cudaMemsetAsync(b->d_perr, 0, (size_t)np * 8, st);
-        rc = elements_run_modes(b->el, b->d_cell_prob, b->d_node_prob, b->d_pmode, b->d_ddu, b->d_ff, b->d_csr, &q,
-                                b->d_perr);
+        rc = elements_run_modes(b->el, b->d_cell_prob, b->d_pmode, b->d_ddu, b->d_ff, b->d_csr, &q, b->d_perr);
         if (rc) return rc;
         cudaMemcpyAsync(b->d_active, elem.data(), np, cudaMemcpyHostToDevice, st);
         residual_kernel<<<(unsigned)b->nchunk, CHN, 0, st>>>(b->S, b->d_ff, b->d_fext, b->d_u, b->d_lam, b->d_c,
@@ -2422,7 +2416,7 @@ int timing_setup(pms_batch* b) {
     if (rc) return rc;
     std::vector<uint8_t> all(np, 1);
     cudaMemcpyAsync(b->d_pmode, all.data(), np, cudaMemcpyHostToDevice, st);
-    rc = elements_run_modes(b->el, b->d_cell_prob, b->d_node_prob, b->d_pmode, b->d_ddu, b->d_ff, b->d_csr);
+    rc = elements_run_modes(b->el, b->d_cell_prob, b->d_pmode, b->d_ddu, b->d_ff, b->d_csr);
     if (rc) return rc;
     rc = elements_status(b->el);
     if (rc) return rc;
