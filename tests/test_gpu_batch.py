@@ -339,3 +339,26 @@ def test_batches_on_each_device():
         th.start()
         th.join()
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("sizes", [[(1, 1, 1)], [(2, 3, 2), (5, 4, 6), (3, 3, 3)], [(8, 9, 7), (2, 2, 2), (16, 10, 12), (4, 5, 6)],
+                                   [(11, 11, 11)] * 9], ids=["one cell", "uneven", "teams and batch-wide", "past the line"])
+def test_batch_wide_engines_in_3d(sizes):
+    """The 3D form of the cooperative kernel (16 lanes a node, one quarter at a time): one problem of eight nodes,
+    several of uneven size, one too large for a team beside smaller ones, and a batch of more than 104 chunks:
+    the iterates and the failures of the teams (the load steps are coarse, and some do not converge),
+    host-sequenced and with the Newton loop on the device."""
+    from pmsim_b200.batch import BatchSolver
+    from pmsim_b200.footing import block_problem
+    probs = [block_problem(*n, 1e4 * (1 + 0.1 * i), 9.0 + i, nsteps=2, hh=500.0) for i, n in enumerate(sizes)]
+    out = []
+    for mode in ("teams", "wide", "device"):
+        b = BatchSolver(probs)
+        if mode == "wide":
+            b.set_tuning(**{**b.tuning(), "team_max_ndof": 0})
+        b.solve(device_loop=mode == "device", on_fail="drop")
+        out.append((b.u(), *b.elements.get_state(), b.history, b.pcg_history, b.failed))
+    for o in out[1:]:
+        for x, y in zip(out[0][:4], o[:4]):
+            assert np.array_equal(x, y)
+        assert out[0][4:] == o[4:]
