@@ -16,7 +16,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpms_b200.so")
 SOURCES = ["pms_material.cu", "pms_plasticity.cu", "pms_elements.cu", "pms_elements3.cu", "pms_gather.cu", "pms_solver.cu", "pms_dpcg.cu", "pms_shapes.cpp", "pms_pattern.cpp"]
-HEADERS = ["pms_device.cuh", "pms_element.cuh", "pms_gather.h", "pms_internal.h", "pms_per_device.h", "pms_shapes.h", "pms_pattern.h"]
+HEADERS = ["pms_device.cuh", "pms_element.cuh", "pms_gather.h", "pms_host_copy.h", "pms_internal.h", "pms_per_device.h", "pms_shapes.h", "pms_pattern.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

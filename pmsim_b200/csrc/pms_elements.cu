@@ -47,6 +47,7 @@
 #include "pms_device.cuh"
 #include "pms_element.cuh"
 #include "pms_gather.h"
+#include "pms_host_copy.h"
 #include "pms_internal.h"
 #include "pms_pattern.h"
 #include "pms_shapes.h"
@@ -1669,7 +1670,7 @@ __global__ void zero_lambda_kernel(int64_t nip, double* lam) {
 // call that finds it in use copies without it), made on first use and kept until exit.
 struct HostStage {
     static constexpr int NSLOT = 4;
-    static constexpr size_t SLOT = size_t(2) << 20;
+    static constexpr size_t SLOT = STAGE_PIECE;
     std::mutex mu;
     char* buf = nullptr;
     bool refused = false;
@@ -2412,6 +2413,15 @@ static int ensure_gather(pms_elements* h) {
     return PMS_OK;
 }
 
+// Host threads that move the pieces of a staged copy on (one within a parallel region of the caller's).
+static int copy_threads() {
+#ifdef _OPENMP
+    return omp_in_parallel() ? 1 : std::max(1, std::min(8, omp_get_max_threads()));
+#else
+    return 1;
+#endif
+}
+
 static bool is_pageable(const void* p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -2422,10 +2432,10 @@ static bool is_pageable(const void* p) {
 }
 
 // The CSR values to pageable memory: pieces of a slot's size come down on the copy stream (each after
-// the slabs it holds are gathered), NSLOT under way at once, and up to eight host threads move a piece
+// the slabs it holds are gathered), NSLOT under way at once, and nt host threads (up to eight) move a piece
 // on while the next ones arrive.  The driver's own copy to pageable memory runs on one thread at 17 GB/s;
 // 45 MB of a 16x15x9 Hex20 block's values took 2.6 of the call's 2.75 ms.
-static bool staged_copy(pms_elements* h, double* csr, const double* d_csr, char* slots) {
+static bool staged_copy(pms_elements* h, double* csr, const double* d_csr, char* slots, int nt) {
     constexpr int NS = pms_elements::NSLAB, NQ = HostStage::NSLOT;
     const size_t total = (size_t)public_nnz(h) * 8, piece = HostStage::SLOT;
     const int64_t npiece = (int64_t)((total + piece - 1) / piece);
@@ -2441,11 +2451,6 @@ static bool staged_copy(pms_elements* h, double* csr, const double* d_csr, char*
     };
     bool ok = true;
     for (int64_t i = 0; i < std::min<int64_t>(NQ, npiece) && ok; i++) ok = issue(i);
-#ifdef _OPENMP
-    const int nt = std::min(8, omp_get_max_threads());
-#else
-    const int nt = 1;
-#endif
     for (int64_t i = 0; i < npiece && ok; i++) {
         ok = cudaEventSynchronize(h->stage_ev[i % NQ]) == cudaSuccess;
         if (!ok) break;
@@ -2522,8 +2527,8 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
     }
     // host CSR: gather NSLAB row slabs; each slab's values go out on the copy stream as soon as
     // the slab is written, overlapping the transfer with the later slabs (and R).  Values for pageable
-    // memory go through the pinned slots (staged_copy); without them, or for pinned memory, the slabs
-    // are copied as they are.
+    // memory go through the pinned slots where that pays (pieces_pay, staged_copy); otherwise, without slots, or
+    // for pinned memory, the slabs are copied as they are.
     if (!h->copy_stream) {
         if (cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking) != cudaSuccess)
             return fail(h, PMS_ERR_CUDA, "stream creation failed");
@@ -2537,7 +2542,8 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
     constexpr int NS = pms_elements::NSLAB;
     std::unique_lock<std::mutex> stage(g_host_stage.mu, std::defer_lock);
     char* slots = nullptr;
-    if (public_nnz(h) * 8 >= (int64_t)HostStage::SLOT && is_pageable(csr) && stage.try_lock()) slots = g_host_stage.slots();
+    const int nt = copy_threads();
+    if (pieces_pay((size_t)public_nnz(h) * 8, nt) && is_pageable(csr) && stage.try_lock()) slots = g_host_stage.slots();
     timed(2, [&] {
         for (int k = 0; k < NS; k++) {
             const int64_t A0 = h->npoint * k / NS, A1 = h->npoint * (k + 1) / NS;
@@ -2552,7 +2558,7 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
     });
     int rc = cuda_check(h);
     if (rc) return rc;
-    if (slots && !staged_copy(h, csr, d_csr, slots)) return cuda_check(h) ? PMS_ERR_CUDA : fail(h, PMS_ERR_CUDA, "copy failed");
+    if (slots && !staged_copy(h, csr, d_csr, slots, nt)) return cuda_check(h) ? PMS_ERR_CUDA : fail(h, PMS_ERR_CUDA, "copy failed");
     if (dof) cudaMemcpyAsync(ff, d_ff, (size_t)h->ndof * 8, cudaMemcpyDeviceToHost, h->stream);
     cudaEventRecord(h->slab_ev[NS], h->copy_stream);
     cudaStreamWaitEvent(h->stream, h->slab_ev[NS], 0);
