@@ -24,6 +24,7 @@ struct ElemArgs {
     int64_t cell0;     // first cell of this launch
     int axisym = 0;    // 2D axisymmetric idealization (x = radius)
     bool overlap = false;  // host side: launch beside the end of the previous kernel (launch_overlapped)
+    int64_t* grid = nullptr;  // host side: receives the blocks launched
     int64_t nip;       // total IPs of the mesh (SoA stride)
     int ngauss;
     double thickness;

@@ -238,10 +238,7 @@ element_kernel(ElemArgs A) {
             Ns[m * 32 + p] = A.tab[ng * NE + ng + i];
         }
     __syncthreads();
-    if constexpr (!CSR) {
-        let_next_start();
-        wait_for_previous();
-    }
+    if constexpr (!CSR) wait_for_previous();
 
     // the warps of one cell meet at a named barrier (id 1 + cell slot)
     auto cell_sync = [&]() {
@@ -1023,10 +1020,7 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
             Ns[m * 16 + p] = A.tab[ng * NE + ng + i];
         }
     __syncthreads();
-    if constexpr (!CSR) {
-        let_next_start();
-        wait_for_previous();
-    }
+    if constexpr (!CSR) wait_for_previous();
 
     // this lane's tile (ti <= tj), row-major over the upper triangle of node groups
     int ti = -1, tj = -1;
@@ -1620,9 +1614,9 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
 template <int ND>
 __global__ void __launch_bounds__(256) f_gather_kernel(int64_t npoint, const int64_t* __restrict__ inc_ptr,
                                                        const int32_t* __restrict__ inc,
-                                                       const double* fe, double* ff) {
-    let_next_start();
+                                                       const double* fe, double* ff, int signal) {
     wait_for_previous();
+    let_next_start(signal);
     for (int64_t A = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; A < npoint;
          A += (int64_t)gridDim.x * blockDim.x) {
         double s[ND];
@@ -1729,7 +1723,7 @@ struct pms_elements {
     int32_t* d_indices = nullptr;
     int32_t* d_status = nullptr;
     int64_t device_bytes = 0;
-    int device = 0;  // its memory and its own stream are there
+    int device = 0, sms = 0;  // its memory and its own stream are there; that device's SMs
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
     std::string last_error;
@@ -1894,6 +1888,7 @@ void launch_elem2d_lpc(pms_elements* h, const ElemArgs& a, cudaStream_t st) {
         kern<<<(unsigned)std::max<int64_t>(blocks, 1), WPB2 * 32, smem, st>>>(a);
     } else {
         void* args[] = {(void*)&a};
+        if (a.grid) *a.grid = blocks;
         launch_overlapped(a.overlap, (const void*)kern, std::max<int64_t>(blocks, 1), WPB2 * 32, smem, st, args);
     }
 }
@@ -1925,6 +1920,7 @@ void launch_elem_t(pms_elements* h, const ElemArgs& a) {
         kern<<<(unsigned)blocks, WPB * 32, h->smem_bytes, h->stream>>>(a);
     } else {
         void* args[] = {(void*)&a};
+        if (a.grid) *a.grid = blocks;
         launch_overlapped(a.overlap, (const void*)kern, blocks, WPB * 32, h->smem_bytes, h->stream, args);
     }
 }
@@ -2054,8 +2050,9 @@ bool gather_is_one_wave(pms_elements* h) {
 }
 
 // CSR gather of the block rows [node0, node0 + nrow) into the handle's storage of the values, and
-// their rows of R (ff, nullable)
-void launch_kk_gather(pms_elements* h, double* csr, double* ff, int64_t node0, int64_t nrow) {
+// their rows of R (ff, nullable).  before: blocks of the element kernel that was launched before it, 0 for a
+// slab after the first
+void launch_kk_gather(pms_elements* h, double* csr, double* ff, int64_t node0, int64_t nrow, int64_t before) {
     GatherArgs P;
     P.node0 = node0;
     P.nrow = nrow;
@@ -2080,14 +2077,17 @@ void launch_kk_gather(pms_elements* h, double* csr, double* ff, int64_t node0, i
         resident = launch_plan(h, g.kern, g.smem, 32 * g.wpb, false);
     }
     const int64_t blocks = std::min(want, resident);
+    P.signal = before + blocks <= h->sms;
     void* args[] = {&P};
     launch_overlapped(want <= resident, g.kern, std::max<int64_t>(blocks, 1), 32 * g.wpb, g.smem, h->stream, args);
     h->launches++;
 }
 
-void launch_f_gather(pms_elements* h, double* ff) {
+// before: blocks of the element kernel that was launched before it
+void launch_f_gather(pms_elements* h, double* ff, int64_t before) {
     int64_t n = h->npoint;
-    void* args[] = {&n, &h->d_inc_ptr, &h->d_inc, &h->d_fe, &ff};
+    int signal = before + grid_1d(n) <= h->sms;
+    void* args[] = {&n, &h->d_inc_ptr, &h->d_inc, &h->d_fe, &ff, &signal};
     launch_overlapped(gather_is_one_wave(h), h->nd == 2 ? (const void*)f_gather_kernel<2> : (const void*)f_gather_kernel<3>, grid_1d(n), 256, 0,
                       h->stream, args);
     h->launches++;
@@ -2152,6 +2152,7 @@ int pms_elements_create(const pms_mesh* mesh, const pms_material* materials, int
     }
     auto* h = new pms_elements();
     cudaGetDevice(&h->device);
+    cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
     h->kind = kind;
     h->nd = mesh->ndim;
     h->nc = 2 * h->nd;
@@ -2494,7 +2495,9 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
         if (rc) return rc;
     }
     ElemArgs a = make_args(h, d_ddu);
+    int64_t before = 0;  // blocks of the element kernel
     a.overlap = !direct && (dof || dok) && gather_is_one_wave(h);
+    a.grid = &before;
     if (direct) {
         a.csr = d_csr;
         a.ff = d_ff;
@@ -2511,10 +2514,10 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
         h->ev_pending[k].push_back(e);
     };
     if (upd != UPD_NONE || dof || dok) timed(0, [&] { launch_elem(h, a, upd, dof, dok, direct); });
-    if (dof && !dok && !direct) timed(1, [&] { launch_f_gather(h, d_ff); });
+    if (dof && !dok && !direct) timed(1, [&] { launch_f_gather(h, d_ff, before); });
     double* k_ff = dof ? d_ff : nullptr;  // R comes out of the row gather of K where both are asked for
     if (mem == PMS_MEM_DEVICE || !dok || direct) {
-        if (dok && !direct) timed(2, [&] { launch_kk_gather(h, d_csr, k_ff, 0, h->npoint); });
+        if (dok && !direct) timed(2, [&] { launch_kk_gather(h, d_csr, k_ff, 0, h->npoint, before); });
         int rc = cuda_check(h);
         if (rc) return rc;
         if (mem == PMS_MEM_HOST) {
@@ -2547,7 +2550,7 @@ static int run(pms_elements* h, const double* ddu, double* ff, double* csr, int 
     timed(2, [&] {
         for (int k = 0; k < NS; k++) {
             const int64_t A0 = h->npoint * k / NS, A1 = h->npoint * (k + 1) / NS;
-            if (A1 > A0) launch_kk_gather(h, d_csr, k_ff, A0, A1 - A0);
+            if (A1 > A0) launch_kk_gather(h, d_csr, k_ff, A0, A1 - A0, k == 0 ? before : 0);
             cudaEventRecord(h->slab_ev[k], h->stream);
             if (slots) continue;
             cudaStreamWaitEvent(h->copy_stream, h->slab_ev[k], 0);

@@ -67,7 +67,6 @@ __global__ void __launch_bounds__(WPB3 * 32, 3) element3_kernel(ElemArgs A) {
     }
     for (int i = threadIdx.x; i < ng; i += blockDim.x) ws[i] = A.tab[ng * 3 * NN + i];
     __syncthreads();
-    let_next_start();
     wait_for_previous();
 
     int ti = -1, tj = -1;  // this lane's tile (ti <= tj), row-major over the node groups
@@ -371,6 +370,7 @@ void launch_t(pms_elements* h, const ElemArgs& a, cudaStream_t stream) {
     const int64_t groups = (a.ncell + CPW - 1) / CPW;
     const int64_t blocks = std::min<int64_t>((groups + WPB3 - 1) / WPB3, launch_plan(h, (const void*)kern, smem, WPB3 * 32));
     void* args[] = {(void*)&a};
+    if (a.grid) *a.grid = blocks;
     launch_overlapped(a.overlap, (const void*)kern, std::max<int64_t>(blocks, 1), WPB3 * 32, smem, stream, args);
 }
 

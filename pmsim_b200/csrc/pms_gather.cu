@@ -75,9 +75,9 @@ __global__ void __launch_bounds__(GATHER_WARPS * 32, FEW ? 2 : 3) gather3_kernel
     double* buf = rowbuf + (int64_t)(wid * ROWS + q) * P.nbmax * 9;
     const int64_t step = (int64_t)gridDim.x * wpb * ROWS;
     int64_t r = ((int64_t)blockIdx.x * wpb + wid) * ROWS;  // first row of the warp (of nrow)
-    let_next_start();
     if (r >= P.nrow) return;
     wait_for_previous();
+    let_next_start(P.signal);
     const bool mine = sub < 3;
     for (; r < P.nrow; r += step) {
         const int64_t A = P.node0 + r + q;
@@ -187,9 +187,9 @@ __global__ void __launch_bounds__(GATHER_WARPS * 32, 5) gather2_kernel(GatherArg
     const int g = min(lane / NN, G - 1), b = lane - g * NN;  // the lanes past G*NN: b >= NN, no blocks
     const int64_t step = (int64_t)gridDim.x * wpb * G;
     int64_t r = ((int64_t)blockIdx.x * wpb + wid) * G;  // first row of the warp (of nrow)
-    let_next_start();
     if (r >= P.nrow) return;
     wait_for_previous();
+    let_next_start(P.signal);
     const bool aligned = ((uintptr_t)P.csr & 15) == 0;  // the caller's values may start on an odd 8 bytes
     for (; r < P.nrow; r += step) {
         const int64_t A = P.node0 + r + g;

@@ -7,14 +7,25 @@
 
 namespace pms {
 
-// Programmatic dependent launch: the kernels of a batched call (element kernel, then gather) let the
-// next one's blocks start as soon as their own have, and wait for the previous kernel to finish
-// before they touch its results, so that launch and start-up overlap its end.  What they read of them
-// they read by ordinary loads (no __ldg, no const __restrict__).  Both are no-ops after an ordinary launch.  Only where the gather is one wave (launch_overlapped's `overlap`): 20x10 Qua8
-// step 16.4 -> 11.6 us, 87x48 Qua9 23.8 -> 20.1, 12x10x6 Hex20 51 -> 45; on larger meshes the early gather
-// blocks run at the element kernel's shared-memory carveout, where they miss in L1 (701x350 Qua8 526 ->
-// 864 us).
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Programmatic dependent launch: the kernels of a batched call (element kernel, then gather) may start up beside
+// the end of the one before and wait for it to finish before they touch its results, so that launch and start-up
+// overlap its end.  What they read of them they read by ordinary loads (no __ldg, no const __restrict__).  The
+// wait and the signal are no-ops after an ordinary launch.  Where the gather is one wave (launch_overlapped's
+// `overlap`; the slabs of a host-array call each by its own size).
+//
+// When the next kernel may start: an element kernel gives no signal, so its gather starts as its last blocks leave;
+// a gather signals once its own wait is over, and only where its blocks and the element kernel's fit the SMs side by
+// side (GatherArgs::signal).  A signal before the wait lets a row of future calls settle on the SMs: they take the slots of
+// the running kernel unevenly, and gathers among them run at the element kernel's shared-memory carveout, where they miss in
+// L1.  Calls in a row, us, plain launches | signals before the waits | here: step of 20x10 Qua8 16.5 | 11.6 | 11.0, 60x45
+// 18.5 | 20.0 | 13.9; 9x8x8 Hex20 39.1 | 45.0 | 35.2; 9x8x8 Hex8 22.6 | 21.6 | 18.0, 11x10x10 22.6 | 28.7 | 18.4; 16x15x15
+// Tet4 43.1 | 46.4 | 39.1, without K 25.9 | 43.0 | 21.5.  A gather's signal above that line: 9x8x8 Hex20 43.1 in place of
+// 35.2, 60x45 Qua8 16.8 and 13.9; none below it: 4x3x3 Hex20 30.4 in place of 28.2, 20x10 Qua8 11.5 and 11.0.
+// (predicated, not a branch, and no memory clobber: the signal publishes nothing, and either would keep the compiler from
+// scheduling the loads around it, 1 us of a 2D step)
+__device__ __forceinline__ void let_next_start(int signal) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p griddepcontrol.launch_dependents;\n\t}" ::"r"(signal));
+}
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 inline cudaError_t launch_overlapped(bool overlap, const void* kern, int64_t blocks, int threads, int smem,
@@ -54,6 +65,7 @@ struct GatherArgs {
     const double* fe;     // [cell][node][ND]
     double* csr;
     double* ff;  // nullable: no R
+    int signal;  // let the next kernel's blocks start beside this one's
     // triangle storages (sym = PMS_SYM_LOWER: columns <= row, PMS_SYM_UPPER: columns >= row;
     // src/base/assembly.rs:92-122): the other entries are not written out, and row (A, i) starts at
     // tbase[A] plus the lengths of rows (A, 0..i-1); kdiag[A] = A's own position in its block row

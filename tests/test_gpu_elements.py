@@ -397,8 +397,9 @@ def test_gather_of_few_rows(kind, ngauss, n, sym):
 
 
 @pytest.mark.parametrize("kind,ngauss,n", [(M.QUA8, 9, (20, 10, 1)), (M.TRI6, 3, (9, 8, 1)), (M.TET4, 4, (4, 3, 3)),
-                                           (M.HEX8, 8, (6, 5, 5)), (M.HEX20, 27, (3, 3, 2))],
-                         ids=["qua8", "tri6", "tet4", "hex8", "hex20"])
+                                           (M.HEX8, 8, (6, 5, 5)), (M.HEX20, 27, (3, 3, 2)),
+                                           (M.QUA8, 9, (60, 45, 1)), (M.TET4, 4, (13, 13, 12)), (M.HEX8, 8, (11, 10, 10))],
+                         ids=["qua8", "tri6", "tet4", "hex8", "hex20", "qua8 more blocks than SMs", "tet4 more", "hex8 more"])
 def test_calls_that_follow_one_another_without_a_wait(kind, ngauss, n):
     """On small meshes the kernels of successive calls overlap their launches while the element matrices are
     written again and again: K and R of many calls in a row, each with another increment (and F_int alone
