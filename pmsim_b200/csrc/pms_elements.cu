@@ -981,6 +981,11 @@ template <int NN, int LPC, int UPD, bool DOF, bool DOK, bool CSR>
 __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
     constexpr int NE = 2 * NN, GS = NE + 2;
     constexpr int CPW = 32 / LPC;  // cells per warp
+    // N/r of every node and point kept by phase 1: where K_e reads it, and for F_e of the larger cells.  The division
+    // unrolled over the nodes costs the kernels that need little else (plane strain too): 420x400 Tri3 F alone 61.3 us
+    // with it, 49.2 with N/r formed by the node's lane, update alone 73.8 and 63.6, Qua4 47.6 and 40.0, Tri6 92.5 and
+    // 86.6, but Qua8 (9 points) 86.5 and 94.3, (4) 69.7 and 71.8.
+    constexpr bool KEEP_Q = DOK || (DOF && NN >= 8);
     using TL = Tile2<NN>;
     constexpr int T = TL::T;
     static_assert(TL::NT <= LPC && NN <= LPC && LPC <= 16, "every node and node-pair tile needs a lane of the cell");
@@ -1164,7 +1169,7 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
                     g[i] = v;
                 }
                 reinterpret_cast<double2*>(Gp)[m] = make_double2(g[0], g[1]);
-                if (A.axisym) Q[p * NN + m] = Ns[m * 16 + p] / rad;  // N/r
+                if (KEEP_Q && A.axisym) Q[p * NN + m] = Ns[m * 16 + p] / rad;  // N/r
                 if (do_update) {
                     const double2 u = U2[m];
                     D[0] = fma(u.x, g[0], D[0]);
@@ -1187,6 +1192,7 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
                 double2* c6 = reinterpret_cast<double2*>(CS + p * 6);
                 c6[0] = make_double2(coef * sig[0], coef * sig[1]);
                 c6[1] = make_double2(coef * sig[3] * INV_SQRT2, coef * sig[2]);
+                if (!KEEP_Q) CS[p * 6 + 4] = rad;
             }
             if (dok_c) {
                 double a, b, s[4];
@@ -1248,7 +1254,7 @@ __global__ void __launch_bounds__(WPB2 * 32, 4) element2d_kernel(ElemArgs A) {
                 const double2 g = reinterpret_cast<const double2*>(G + p * GS)[hl];
                 f[0] += d.x * g.x + o.x * g.y;
                 f[1] += o.x * g.x + d.y * g.y;
-                if (A.axisym) f[0] += o.y * Q[p * NN + hl];
+                if (A.axisym) f[0] += o.y * (KEEP_Q ? Q[p * NN + hl] : Ns[hl * 16 + p] / CS[p * 6 + 4]);
             }
             if (CSR) {  // kept in the cell's dU slot (free after phase 1) until the scatter
                 Us[hl * 2] = f[0];
