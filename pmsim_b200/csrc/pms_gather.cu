@@ -18,9 +18,10 @@ constexpr unsigned FULL = 0xffffffffu;
 // is resident while they are written, and the read-only path (__ldg) is for memory that stays as it is from
 // the kernel's start to its end; the maps of the mesh do.
 //
-// Bounds: 64x64x32 Hex20 moves 4.2 GB (0.65 ms at 6.5 TB/s) and takes 1.57 ms, as before with a lane per
-// 3x3 block: the LSU data pipe (each 8-byte value is loaded, added in shared memory and written out)
-// and the row's chain of dependent loads.  The other kinds gained: 40x40x40 Hex8 136 -> 116 us (lower
+// Bounds: 64x64x32 Hex20 moves 4.2 GB (0.65 ms at 6.5 TB/s) and takes 1.54 ms, a lane per 3x3 block took 1.57:
+// the LSU data pipe (each 8-byte value is loaded, added in shared memory and written out; busy 72% on 32x32x16
+// Hex20, 84% on 40x40x40 Hex8, 83% on 350x350 Qua8, 66% on 24x23x21 Tet4) and the row's chain of dependent
+// loads (long scoreboard: 39, 44, 68 and 52% of the cycles between a warp's instructions).  The other kinds gained: 40x40x40 Hex8 136 -> 116 us (lower
 // triangle 136 -> 114), 701x350 Qua8 231 -> 176, 24x23x21 Tet4 60 -> 50, 400x300 Tri6 151 -> 110,
 // 20x10 Qua8 15 -> 8.6 us (F_int and K in one launch).  Measured slower: ranges and incidences loaded a
 // row or two ahead (Hex20 1.9 ms, 701x350 Qua8 0.46 ms: fewer warps, spills), source lists per block of K with the
@@ -49,16 +50,17 @@ template <int NN> struct Gather3 {
     static constexpr int ROWS = NN >= 13 ? 1 : 3;
     static constexpr int BPI = 3 / ROWS;              // blocks at a time
     static constexpr int NIT = (NN + BPI - 1) / BPI;  // blocks per lane and incidence
-    static constexpr bool FEW = NN != 10;             // has a kernel for few rows (no mesh of Tet10 to measure)
+    static constexpr bool FEW = NN < 10;              // has a kernel for few rows
     static constexpr int CL = ROWS == 1 ? 27 : 9;     // lanes that hold a row's incidences
 };
 
 // NB incidences are loaded before they are added: two with one row a warp, one with three rows (the registers
-// of two cost a third of the warps: 40x40x40 Hex8 255 us a step with one, 266 with two).  Where the call's
-// rows are all in flight at once anyway (FEW), the chain of a row's loads is the time: the warps get more
-// registers and load two incidences ahead (four for Tet4, whose rows are up to 24 cells long).  First K
-// of 17x18x15 Hex8 49.2 -> 39.6 us, 6x6x6 Tet4 33.6 -> 29.3, 6x6x6 Hex20 45.5 -> 39.7; four incidences for Hex8
-// or Hex20 gave the same as two.
+// of two cost a third of the warps: 40x40x40 Hex8 255 us a step with one, 266 with two; Tet4, with half the blocks a
+// lane, was not measured beyond few rows).  Where the call's rows are all in flight at once anyway (FEW), the chain of
+// a row's loads is the time: the warps get more registers and load two incidences ahead (four for Tet4, whose rows are
+// up to 24 cells long).  K in calls that follow one another, us: Hex8 5x5x5 14.5 -> 13.1, 9x8x8 15.6 -> 14.1, 13x13x12
+// 17.9 -> 16.6, 17x18x15 22.8 and 22.8; Tet4 6x6x6 21.3 -> 16.7, 13x13x12 25.9 -> 21.0, 18x18x18 38.9 -> 36.0.  Hex20
+// gains nothing (6x6x6 21.0 and 21.0), Tet10 was not measured.  Four incidences for Hex8 gave the same as two.
 template <int NN, bool TRI, bool FEW>
 __global__ void __launch_bounds__(GATHER_WARPS * 32, FEW ? 2 : 3) gather3_kernel(GatherArgs P) {
     constexpr int NU = NN * (NN + 1) / 2;

@@ -75,7 +75,7 @@ struct GatherArgs {
 };
 
 // Kernel and launch shape of an element kind's gather; few: the kernel for calls whose rows are all in
-// flight at once, where the kind has one (Tet4, Hex8, Hex20).
+// flight at once, where the kind has one (Tet4, Hex8).
 struct GatherShape {
     const void* kern;
     int rows;  // block rows per warp
