@@ -7,7 +7,8 @@
 // upper triangle (K_e).  Phase 1 leaves the gradients g and, at plastic points, h = S g of every node
 // in shared memory, so the pairs read both with 16-byte loads and no barrier.
 //
-// Bounds: FP64 latency at 12 warps (36 Hex8 or 96 Tet4 cells) per SM; 16 warps spill.  Element kernel of a
+// Bounds: the shared-memory data path (LSU data pipe busy 83% on 40x40x40 Hex8, FP64 pipe 34%) at 12 warps (36
+// Hex8 or 96 Tet4 cells) per SM; 16 warps spill.  Element kernel of a
 // fused step: 40x40x40 Hex8 326 us with a warp per cell, 147 us here (2 blocks per SM 166, 4 blocks 165);
 // 30x30x30 Tet4 squares (162,000 cells) 378 and 132 us.  Larger cells (Tet10: 15 tiles, Hex20) stay with
 // a warp per cell, and so do rules with more points than lanes per cell (Hex8 with 27).

@@ -343,7 +343,7 @@ __device__ __forceinline__ int ep_select(const MatConst& m, const EpConst& e, do
 // warp w of nwarp owns the runs of 32 IPs w, w + nwarp, ... and hands out their IPs in order, once
 // REFILL lanes are idle (the selection costs about as much as a step, for one lane or for 32;
 // REFILL = 4, 8 and 12 measured 1.44, 1.45 and 1.49 ms, no refill before all are done 2.15 ms).
-// Bound by the FP64 pipe and its latency: about 330 instructions a step, 12 warps per SM in 3D (168
+// Bound by the FP64 pipe (49% busy in 3D) and its latency: about 330 instructions a step, 12 warps per SM in 3D (162
 // registers; 16 warps with spills and 10 without measured the same or slower), 16 in 2D.
 // 1,048,576 IPs, half of them on the yield surface, the others inside it: 28.4 ms in 3D and 5.3 ms in
 // 2D with all stress components integrated, one IP a thread; 1.45 and 0.88 ms here.  4,000 3D IPs:

@@ -518,6 +518,8 @@ pcg_beta_direction_kernel(SolverArgs S, int par, const double* part_rz, const do
 //   -- barrier -- alpha from the partials (every block of a problem sums the same ones in the same order)
 //   B  x, r, z of the own quarters, partials of r.z and r.r
 //   -- barrier -- beta, iteration count and stopping test from the partials
+// p = z + beta p' is formed at prescribed DOFs too, where both are 0 unless the residual has overflowed: such a
+// problem fails on every engine, with other entries infinite or NaN.
 // Bound by the barriers (2.3 to 3 us each, L2 round trips) and the dependent loads of a phase.  Time of an
 // iteration, three kernels in a CUDA graph and this: 661 nodes (20x10 Qua8) 13.9 and 10.3 us, 1,331 (10x10x10 Hex8)
 // 14.1 and 10.9, 9,261 (20^3) 14.6 and 13.4, six footings of 13,236 14.9 and 14.1; but 15,425 15.0 and 17.4,
