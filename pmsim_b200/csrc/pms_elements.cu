@@ -935,9 +935,9 @@ element_kernel(ElemArgs A) {
 // at the plastic points, so phase 2 reads its operands from shared memory with no per-point staging
 // or barrier.  Every entry of K_e takes the same operations in the same order as in element_kernel.
 // The kernel is bound by the shared-memory data path (the LSU data pipe busy 80% at 122,500 plane-strain Qua8
-// cells, the FP64 pipe 39%; 82% before what follows), so operands are read as pairs, strains come from the displacement gradient, and h is neither formed
-// nor stored where nothing reads it: 354 -> 340 us at 245,350 cells, and 41.0 -> 39.7 us for the step of 12,960
-// axisymmetric Qua8 cells.  A slot without a cell (ragged end, inactive problem) repeats the
+// cells, the FP64 pipe 39%; 82% before what follows), so operands are read as pairs, strains come from the
+// displacement gradient, and h is neither formed nor stored where nothing reads it: 354 -> 340 us at 245,350
+// cells, and 41.0 -> 39.7 us for the step of 12,960 axisymmetric Qua8 cells.  A slot without a cell (ragged end, inactive problem) repeats the
 // group's first cell and writes nothing: all slots run the same loop trips, so the warp-wide syncs
 // below are always reached by all 32 lanes.
 constexpr int WPB2 = 4;      // warps per block
